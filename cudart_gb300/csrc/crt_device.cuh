@@ -174,22 +174,20 @@ extern __shared__ float4 crt_top_nodes[];
 
 // Per-thread stack: shared-memory part (stride = threads per block) and a
 // local-memory overflow part.  It also carries how many top nodes the
-// launching kernel staged in shared memory (0: none).
+// launching kernel staged in shared memory (0: none).  The overflow array is
+// the kernel's own variable: as a member, its dynamic indexing would keep the
+// whole struct, the stack pointer included, in local memory.
+using StackSpill = uint2[kMaxLevels];
 struct Stack {
     uint2* sh;           // this thread's first shared entry; entries are `stride` apart
+    uint2* spill;
     uint32_t stride;     // threads per block
     int depth;           // entries kept in shared memory
     int sp;
-    uint32_t n_top = 0;  // nodes [0, n_top) are in crt_top_nodes
-    uint2 spill[kMaxLevels];
+    uint32_t n_top;      // nodes [0, n_top) are in crt_top_nodes
 
-    CRT_D void setup(uint2* base, uint32_t threads, int shared_depth, uint32_t staged_nodes = 0) {
-        sh = base + threadIdx.x;
-        stride = threads;
-        depth = shared_depth;
-        sp = 0;
-        n_top = staged_nodes;
-    }
+    CRT_D Stack(uint2* base, StackSpill& overflow, uint32_t threads, int shared_depth, uint32_t staged_nodes = 0)
+        : sh(base + threadIdx.x), spill(overflow), stride(threads), depth(shared_depth), sp(0), n_top(staged_nodes) {}
     CRT_D void push(uint2 e) {
         if (sp < depth) sh[sp * stride] = e;
         else spill[sp - depth] = e;

@@ -31,8 +31,8 @@ template <bool F32>
 #endif
 __global__ void __maxnreg__(F32 ? CRT_MEGA_REGS + 16 : CRT_MEGA_REGS) mega_kernel(RenderParams P) {
     __shared__ uint2 stack_sh[kStackShared * kMegaBlock];
-    Stack st;
-    st.setup(stack_sh, kMegaBlock, kStackShared);
+    StackSpill overflow;
+    Stack st(stack_sh, overflow, kMegaBlock, kStackShared);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t x = blockIdx.x * 16u + (warp & 1u) * 8u + (lane & 7u);
     const uint32_t y = blockIdx.y * 8u + (warp >> 1) * 4u + (lane >> 3);

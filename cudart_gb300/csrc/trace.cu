@@ -18,8 +18,8 @@ __global__ void __launch_bounds__(kTraceBlock) trace_closest_kernel(DevScene S, 
                                                                     uint32_t* __restrict__ out_nodes,
                                                                     uint32_t* __restrict__ out_tris) {
     __shared__ uint2 stack_sh[kStackShared * kTraceBlock];
-    Stack st;
-    st.setup(stack_sh, kTraceBlock, kStackShared);
+    StackSpill overflow;
+    Stack st(stack_sh, overflow, kTraceBlock, kStackShared);
     for (uint32_t i = blockIdx.x * kTraceBlock + threadIdx.x; i < n; i += gridDim.x * kTraceBlock) {
         const float4 a = rays[2ull * i], b = rays[2ull * i + 1];
         Hit h;

@@ -485,8 +485,8 @@ CRT_D uint2* stage_top_nodes(const WaveParams& W) {
 template <bool REFILL, bool WHOLE_LEAF, bool F32, bool TOP>
 __global__ void __maxnreg__(F32 ? CRT_TRAVERSAL_REGS_F32 : CRT_TRAVERSAL_REGS) wf_extend(WaveParams W) {
     uint2* stacks = stage_top_nodes<F32, TOP>(W);
-    Stack st;
-    st.setup(stacks, blockDim.x, W.stack_depth, TOP ? W.top_nodes : 0u);
+    StackSpill overflow;
+    Stack st(stacks, overflow, blockDim.x, W.stack_depth, TOP ? W.top_nodes : 0u);
     const uint32_t cur = W.counters[C_CUR];
     __shared__ uint32_t pre_sh[9];
     ExtendJob<WHOLE_LEAF, F32> job(W, queue_view(W, cur, pre_sh), st);
@@ -766,8 +766,8 @@ __global__ void __maxnreg__(F32 ? CRT_TRAVERSAL_REGS_F32 : CRT_TRAVERSAL_REGS) w
     uint2* stacks = stage_top_nodes<F32, true>(W);
     float* grad = reinterpret_cast<float*>(stacks + (size_t)blockDim.x * W.stack_depth);
     zero_grad_block(grad, W.n_mats);
-    Stack st;
-    st.setup(stacks, blockDim.x, W.stack_depth, W.top_nodes);
+    StackSpill overflow;
+    Stack st(stacks, overflow, blockDim.x, W.stack_depth, W.top_nodes);
     ShadowJob<true, F32, true> job(W, st, grad);
     persistent_loop<false>(W.counters[C_SHADOW], &W.counters[C_FETCH_SHD], W.queue_chunk, 31u, job);
     count_rays(W.R.ray_counts, 0, job.rays);
@@ -777,8 +777,8 @@ __global__ void __maxnreg__(F32 ? CRT_TRAVERSAL_REGS_F32 : CRT_TRAVERSAL_REGS) w
 template <bool REFILL, bool WHOLE_LEAF, bool F32, bool TOP>
 __global__ void __maxnreg__(F32 ? CRT_TRAVERSAL_REGS_F32 : CRT_TRAVERSAL_REGS) wf_shadow(WaveParams W) {
     uint2* stacks = stage_top_nodes<F32, TOP>(W);
-    Stack st;
-    st.setup(stacks, blockDim.x, W.stack_depth, TOP ? W.top_nodes : 0u);
+    StackSpill overflow;
+    Stack st(stacks, overflow, blockDim.x, W.stack_depth, TOP ? W.top_nodes : 0u);
     ShadowJob<WHOLE_LEAF, F32> job(W, st);
     persistent_loop<REFILL>(W.counters[C_SHADOW], &W.counters[C_FETCH_SHD], W.queue_chunk, W.refill_busy, job);
     count_rays(W.R.ray_counts, 0, job.rays);
@@ -896,8 +896,8 @@ CRT_D void add_top(unsigned long long* p, uint32_t top) {
 template <bool F32>
 __global__ void __launch_bounds__(kWaveBlock) wf_extend_count(WaveParams W) {
     __shared__ uint2 stack_sh[kStackShared * kWaveBlock];
-    Stack st;
-    st.setup(stack_sh, kWaveBlock, kStackShared);
+    StackSpill overflow;
+    Stack st(stack_sh, overflow, kWaveBlock, kStackShared);
     const uint32_t cur = W.counters[C_CUR];
     const uint32_t n = W.counters[cur];
     __shared__ uint32_t pre_sh[9];
@@ -930,8 +930,8 @@ __global__ void __launch_bounds__(kWaveBlock) wf_extend_count(WaveParams W) {
 template <bool F32>
 __global__ void __launch_bounds__(kWaveBlock) wf_shadow_count(WaveParams W) {
     __shared__ uint2 stack_sh[kStackShared * kWaveBlock];
-    Stack st;
-    st.setup(stack_sh, kWaveBlock, kStackShared);
+    StackSpill overflow;
+    Stack st(stack_sh, overflow, kWaveBlock, kStackShared);
     const uint32_t n = W.counters[C_SHADOW];
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t rays = 0;
