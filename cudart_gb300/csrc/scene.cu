@@ -438,6 +438,8 @@ int crt_scene_create(const crt_scene_desc* d, crt_scene* out) {
     }
     cudaError_t e = s->error.alloc(16);
     if (e == cudaSuccess) e = cudaMemset(s->error.p, 0, 16);
+    // renders run on streams that do not wait for this one
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
     if (e != cudaSuccess) { delete s; return cuda_error(e, "error word"); }
 
     DevScene& D = s->dev;
@@ -486,6 +488,7 @@ int crt_scene_clear_errors(crt_scene s) {
     if (!s) return set_error(CRT_ERR_INVALID, "crt_scene_clear_errors: null scene");
     CRT_CUDA(cudaDeviceSynchronize());
     CRT_CUDA(cudaMemset(s->error.p, 0, 16));
+    CRT_CUDA(cudaStreamSynchronize(nullptr));   // the next pass may be on any stream
     return CRT_OK;
 }
 
@@ -515,6 +518,7 @@ int crt_scene_set_materials(crt_scene s, const crt_material* materials, uint32_t
     CRT_CUDA(cudaSetDevice(s->device));
     CRT_CUDA(cudaDeviceSynchronize());   // no queued pass may read a half-written table
     CRT_CUDA(cudaMemcpy(s->mats.p, mats.data(), mats.size() * sizeof(float4), cudaMemcpyHostToDevice));
+    CRT_CUDA(cudaStreamSynchronize(nullptr));   // the next pass may be on any stream
     return CRT_OK;
 }
 

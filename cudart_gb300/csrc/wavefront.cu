@@ -1028,7 +1028,10 @@ static bool window_sort(uint32_t flags) {
     return !(flags & (CRT_FLAG_NO_WINDOW_SORT | CRT_FLAG_OCTANT_QUEUES));
 }
 
-static int alloc_set(WaveSet& S, uint32_t cap, bool octant) {
+// `ready`: the stream the set's first use follows (the handle's).  The
+// counters are cleared there: a memset on the default stream could run after
+// the set's first kernels had started, which do not wait for that stream.
+static int alloc_set(WaveSet& S, uint32_t cap, bool octant, cudaStream_t ready) {
     WaveBuffers& B = S.buf;
     B.capacity = cap;
     B.octant = octant;
@@ -1041,7 +1044,7 @@ static int alloc_set(WaveSet& S, uint32_t cap, bool octant) {
     CRT_CUDA(B.shadow.alloc(c * 48));
     CRT_CUDA(B.shadow_q.alloc(c * 4));
     CRT_CUDA(B.counters.alloc(C_COUNT * 4));
-    CRT_CUDA(cudaMemset(B.counters.p, 0, C_COUNT * 4));
+    CRT_CUDA(cudaMemsetAsync(B.counters.p, 0, C_COUNT * 4, ready));
     CRT_CUDA(B.waves.alloc(kMaxWaves * sizeof(uint4)));
     B.seg_capacity = kMaxWaves;
     CRT_CUDA(B.segs.alloc((size_t)B.seg_capacity * sizeof(WaveSeg)));
@@ -1063,7 +1066,7 @@ static int ensure_wave_sets(crt_render r, uint32_t count) {
     CRT_CUDA(cudaEventCreateWithFlags(&r->pass_start, cudaEventDisableTiming));
     r->sets.resize(count);
     for (WaveSet& s : r->sets) {
-        int st = alloc_set(s, cap, octant);
+        int st = alloc_set(s, cap, octant, r->stream);
         if (st != CRT_OK) {
             destroy_wave_sets(r);
             return st;
