@@ -571,15 +571,15 @@ bool build_bvh8(const float* v1, const float* e1, const float* e2, uint32_t n,
                     for (int k = 0; k < 3; ++k) {
                         node.qlo[k][s] = 255;
                         node.qhi[k][s] = 0;
-                        fnode.lo[k][s] = FLT_MAX;
-                        fnode.hi[k][s] = -FLT_MAX;
+                        fnode.planes[k][0][s] = FLT_MAX;
+                        fnode.planes[k][1][s] = -FLT_MAX;
                     }
                     continue;
                 }
                 const Node2& cn = n2[w.ch[c]];
                 for (int k = 0; k < 3; ++k) {
-                    fnode.lo[k][s] = cn.box.lo[k];
-                    fnode.hi[k][s] = cn.box.hi[k];
+                    fnode.planes[k][0][s] = cn.box.lo[k];
+                    fnode.planes[k][1][s] = cn.box.hi[k];
                 }
                 for (int k = 0; k < 3; ++k) {
                     double step = std::ldexp(1.0, e[k]);
@@ -608,9 +608,9 @@ bool build_bvh8(const float* v1, const float* e1, const float* e2, uint32_t n,
                 }
             }
             out.nodes[q] = node;
-            fnode.child_base_imask = node.child_base | ((uint32_t)node.imask << 24);
+            fnode.child_base = node.child_base;
             fnode.tri_base = node.tri_base;
-            std::memcpy(fnode.meta, node.meta, 8);
+            fnode.slots = slots_word(node.imask, node.meta);
             out.fnodes[q] = fnode;
         }
     });

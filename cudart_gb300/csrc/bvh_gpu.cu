@@ -433,22 +433,15 @@ __global__ void k_choose(const int32_t* __restrict__ front, uint32_t F, const GN
     cnt_tri[f] = nt;
 }
 
-__device__ int scale_exponent_d(double ext) {
-    if (!(ext > 0.0)) return -126;
-    int k;
-    const double m = frexp(ext / 255.0, &k);
-    const int e = (m == 0.5) ? k - 1 : k;
-    return max(-126, min(127, e));
-}
-
-// Encodes the wide nodes of one level (the host build's encoding), writes
+// Encodes the wide nodes of one level (both device encodings), writes
 // the next level's frontier and the triangle records of the leaf slots.
 __global__ void k_emit(const GWide* __restrict__ recs, uint32_t F, uint32_t level_base, uint32_t next_base,
                        uint32_t tri_level_base, const uint32_t* __restrict__ int_off,
                        const uint32_t* __restrict__ tri_off, const GNode* __restrict__ nodes,
                        const GDec* __restrict__ dec, const uint32_t* __restrict__ perm, const float* __restrict__ v1,
-                       const float* __restrict__ e1, const float* __restrict__ e2, Bvh8Node* __restrict__ out,
-                       Bvh8FloatNode* __restrict__ fout, TriRecord* __restrict__ tris, int32_t* __restrict__ next_front,
+                       const float* __restrict__ e1, const float* __restrict__ e2, DevNodeQ16* __restrict__ out,
+                       Bvh8FloatNode* __restrict__ fout, DevTriA* __restrict__ tris_a,
+                       DevTriB* __restrict__ tris_b, int32_t* __restrict__ next_front,
                        uint32_t n_tris, uint32_t cap_nodes, uint32_t* err) {
     const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= F) return;
@@ -463,18 +456,15 @@ __global__ void k_emit(const GWide* __restrict__ recs, uint32_t F, uint32_t leve
     GBox nb;
     for (int k = 0; k < 3; ++k) { nb.lo[k] = FLT_MAX; nb.hi[k] = -FLT_MAX; }
     for (int c = 0; c < w.nch; ++c) grow(nb, nodes[w.ch[c]].box);
-    Bvh8Node node;
+    DevNodeQ16 node;
     memset(&node, 0, sizeof(node));
+    clear_planes16(node);
+    uint32_t slots = 0;
     Bvh8FloatNode fnode;
     memset(&fnode, 0, sizeof(fnode));
     node.px = nb.lo[0];
     node.py = nb.lo[1];
     node.pz = nb.lo[2];
-    int e[3];
-    for (int k = 0; k < 3; ++k) e[k] = scale_exponent_d((double)nb.hi[k] - (double)nb.lo[k]);
-    node.ex = (uint8_t)(e[0] + 127);
-    node.ey = (uint8_t)(e[1] + 127);
-    node.ez = (uint8_t)(e[2] + 127);
     node.child_base = next_base + int_off[f];
     node.tri_base = tri_level_base + tri_off[f];
     uint32_t tri_o = 0, int_o = 0;
@@ -482,31 +472,24 @@ __global__ void k_emit(const GWide* __restrict__ recs, uint32_t F, uint32_t leve
         const int c = child_at[s];
         if (c < 0) {
             for (int k = 0; k < 3; ++k) {
-                node.qlo[k][s] = 255;
-                node.qhi[k][s] = 0;
-                fnode.lo[k][s] = FLT_MAX;
-                fnode.hi[k][s] = -FLT_MAX;
+                fnode.planes[k][0][s] = FLT_MAX;
+                fnode.planes[k][1][s] = -FLT_MAX;
             }
             continue;
         }
         const GNode& cn = nodes[w.ch[c]];
         for (int k = 0; k < 3; ++k) {
-            fnode.lo[k][s] = cn.box.lo[k];
-            fnode.hi[k][s] = cn.box.hi[k];
-            const double step = ldexp(1.0, e[k]);
-            const double lo = floor(((double)cn.box.lo[k] - (double)nb.lo[k]) / step);
-            const double hi = ceil(((double)cn.box.hi[k] - (double)nb.lo[k]) / step);
-            node.qlo[k][s] = (uint8_t)fmax(0.0, fmin(255.0, lo));
-            node.qhi[k][s] = (uint8_t)fmax(0.0, fmin(255.0, hi));
+            fnode.planes[k][0][s] = cn.box.lo[k];
+            fnode.planes[k][1][s] = cn.box.hi[k];
+            set_planes16(node, k, s, (double)cn.box.lo[k] - (double)nb.lo[k], (double)cn.box.hi[k] - (double)nb.lo[k]);
         }
         if (wide_slot(dec, w.ch[c])) {
-            node.imask |= (uint8_t)(1u << s);
-            node.meta[s] = 0x80;
+            slots |= 1u << s;
             const uint32_t k = int_off[f] + int_o++;
             if (next_base + k < cap_nodes) next_front[k] = w.ch[c];
             else atomicOr(err, 2u);
         } else {
-            node.meta[s] = (uint8_t)((cn.count << 5) | tri_o);
+            slots |= ((1u << cn.count) - 1u) << (8 + 3 * s);
             // the subtree's triangles, left to right (at most kSlotTrisMax)
             uint32_t pos[kSlotTrisMax];
             uint32_t np = 0;
@@ -531,24 +514,27 @@ __global__ void k_emit(const GWide* __restrict__ recs, uint32_t F, uint32_t leve
             if (np != cn.count) atomicOr(err, 4u);
             for (uint32_t i = 0; i < np; ++i) {
                 const uint32_t t = perm[pos[i]];
-                TriRecord r;
+                DevTriA ra;
                 for (int k = 0; k < 3; ++k) {
-                    r.v1[k] = v1[3ull * t + k];
-                    r.e1[k] = e1[3ull * t + k];
-                    r.e2[k] = e2[3ull * t + k];
+                    ra.v1[k] = v1[3ull * t + k];
+                    ra.e1[k] = e1[3ull * t + k];
                 }
-                r.face = t;
-                r.pad1 = r.pad2 = 0.f;
-                if (node.tri_base + tri_o + i < n_tris) tris[node.tri_base + tri_o + i] = r;
-                else atomicOr(err, 4u);
+                ra.face = t;
+                ra.e2x = e2[3ull * t];
+                if (node.tri_base + tri_o + i < n_tris) {
+                    tris_a[node.tri_base + tri_o + i] = ra;
+                    tris_b[node.tri_base + tri_o + i] = DevTriB{e2[3ull * t + 1], e2[3ull * t + 2]};
+                } else {
+                    atomicOr(err, 4u);
+                }
             }
             tri_o += np;
         }
     }
+    node.slots = fnode.slots = slots;
     out[level_base + f] = node;
-    fnode.child_base_imask = node.child_base | ((uint32_t)node.imask << 24);
+    fnode.child_base = node.child_base;
     fnode.tri_base = node.tri_base;
-    memcpy(fnode.meta, node.meta, 8);
     fout[level_base + f] = fnode;
 }
 
@@ -557,8 +543,8 @@ uint32_t blocks(uint64_t n) { return (uint32_t)std::max<uint64_t>(1, (n + kBlock
 }  // namespace
 
 // Builds the BVH of n triangles (device arrays v1/e1/e2, [n][3]) into nodes,
-// fnodes and tris (device, allocated here); fills max_depth and the node
-// count.  Returns CRT_OK or an error with its message set.
+// fnodes and tris (device, allocated here; tris holds n DevTriA, then n
+// DevTriB); fills max_depth and the node count.  Returns CRT_OK or an error with its message set.
 int build_bvh_gpu(const float* d_v1, const float* d_e1, const float* d_e2, uint32_t n, uint32_t max_levels,
                   int max_children, DevBuf& nodes_out, DevBuf& fnodes_out, DevBuf& tris_out, uint32_t* num_nodes,
                   uint32_t* max_depth, bool* fnodes_ok, cudaStream_t s) {
@@ -664,9 +650,9 @@ int build_bvh_gpu(const float* d_v1, const float* d_e1, const float* d_e2, uint3
 
     // ---- collapse level by level -------------------------------------------
     const uint32_t cap_nodes = n;   // a wide node holds >= 1 triangle of its own subtree
-    CRT_CUDA(nodes_out.alloc((size_t)cap_nodes * sizeof(Bvh8Node)));
+    CRT_CUDA(nodes_out.alloc((size_t)cap_nodes * sizeof(DevNodeQ16)));
     CRT_CUDA(fnodes_out.alloc((size_t)cap_nodes * sizeof(Bvh8FloatNode)));
-    CRT_CUDA(tris_out.alloc((size_t)n * sizeof(TriRecord)));
+    CRT_CUDA(tris_out.alloc((size_t)n * (sizeof(DevTriA) + sizeof(DevTriB))));
     DevBuf front_a, front_b, recs, cnt_int, cnt_tri, off_int, off_tri, scan_tmp;
     CRT_CUDA(front_a.alloc((size_t)cap_nodes * 4));
     CRT_CUDA(front_b.alloc((size_t)cap_nodes * 4));
@@ -697,8 +683,9 @@ int build_bvh_gpu(const float* d_v1, const float* d_e1, const float* d_e2, uint3
         const uint32_t next_base = level_base + F;
         k_emit<<<blocks(F), kBlock, 0, s>>>(recs.as<GWide>(), F, level_base, next_base, tri_base,
                                             off_int.as<uint32_t>(), off_tri.as<uint32_t>(), gn, dec, perm.as<uint32_t>(),
-                                            d_v1, d_e1, d_e2, nodes_out.as<Bvh8Node>(), fnodes_out.as<Bvh8FloatNode>(),
-                                            tris_out.as<TriRecord>(), nxt, n, cap_nodes, err);
+                                            d_v1, d_e1, d_e2, nodes_out.as<DevNodeQ16>(), fnodes_out.as<Bvh8FloatNode>(),
+                                            tris_out.as<DevTriA>(),
+                                            reinterpret_cast<DevTriB*>(tris_out.as<DevTriA>() + n), nxt, n, cap_nodes, err);
         uint32_t totals[2];
         CRT_CUDA(cudaMemcpyAsync(&totals[0], off_int.as<uint32_t>() + F, 4, cudaMemcpyDeviceToHost, s));
         CRT_CUDA(cudaMemcpyAsync(&totals[1], off_tri.as<uint32_t>() + F, 4, cudaMemcpyDeviceToHost, s));

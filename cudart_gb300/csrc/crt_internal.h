@@ -144,10 +144,6 @@ inline uint32_t traversal_block(const crt_render_options& o) { return o.block_si
 inline uint32_t traversal_stack(const crt_render_options& o) { return o.stack_depth ? o.stack_depth : 8u; }
 inline uint32_t queue_chunk(const crt_render_options& o) { return o.queue_chunk ? o.queue_chunk : 32u; }
 inline uint32_t refill_busy(const crt_render_options& o) { return o.refill_busy ? o.refill_busy : 31u; }
-inline uint32_t staged_nodes(const crt_scene_s* s, const crt_render_options& o) {
-    return o.top_nodes < s->info.num_nodes ? o.top_nodes : s->info.num_nodes;
-}
-
 // Default paths in flight per wave set: about 16 samples of every pixel of
 // the handle's views, rounded up to a power of two in [2^16, 2^25] (32M paths
 // at 1080p, 4.7 GB of path state per set).  Longer waves balance the thin

@@ -7,6 +7,7 @@
 // 8-wide quantised tree (bvh8.cpp) instead of two 1-D textures.
 #include "crt_internal.h"
 
+#include <algorithm>
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -43,6 +44,103 @@ int upload(DevBuf& b, const std::vector<T>& v) {
     return CRT_OK;
 }
 
+// Host records to the device layouts.  The 16-bit planes come from the FP32
+// ones where there are any (fnodes), else from the 8-bit ones.
+__global__ void k_pack_bvh(const Bvh8Node* __restrict__ nodes, const Bvh8FloatNode* __restrict__ fnodes,
+                           uint32_t n_nodes, const TriRecord* __restrict__ tris, uint32_t n_tris,
+                           DevNodeQ16* __restrict__ out, DevTriA* __restrict__ ta, DevTriB* __restrict__ tb) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_nodes; i += gridDim.x * blockDim.x) {
+        const Bvh8Node s = nodes[i];
+        DevNodeQ16 d;
+        d.px = s.px; d.py = s.py; d.pz = s.pz;
+        d.child_base = s.child_base;
+        d.tri_base = s.tri_base;
+        d.slots = slots_word(s.imask, s.meta);
+        d.pad[0] = d.pad[1] = 0;
+        clear_planes16(d);
+        const float p[3] = {s.px, s.py, s.pz};
+        const int e[3] = {s.ex, s.ey, s.ez};
+        for (int j = 0; j < 8; ++j) {
+            if (s.meta[j] == 0) continue;
+            for (int k = 0; k < 3; ++k) {
+                const double step = ldexp(1.0, e[k] - 127);
+                const double lo = fnodes ? (double)fnodes[i].planes[k][0][j] - (double)p[k] : s.qlo[k][j] * step;
+                const double hi = fnodes ? (double)fnodes[i].planes[k][1][j] - (double)p[k] : s.qhi[k][j] * step;
+                set_planes16(d, k, j, lo, hi);
+            }
+        }
+        out[i] = d;
+    }
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_tris; i += gridDim.x * blockDim.x) {
+        const TriRecord s = tris[i];
+        ta[i] = DevTriA{{s.v1[0], s.v1[1], s.v1[2]}, s.face, {s.e1[0], s.e1[1], s.e1[2]}, s.e2[0]};
+        tb[i] = DevTriB{s.e2[1], s.e2[2]};
+    }
+}
+
+// Smallest k with ext / 255 <= 2^k, in the range of the exponent byte (the
+// host build's rule).
+__device__ int scale_exponent_d(double ext) {
+    if (!(ext > 0.0)) return -126;
+    int k;
+    const double m = frexp(ext / 255.0, &k);
+    const int e = (m == 0.5) ? k - 1 : k;
+    return max(-126, min(127, e));
+}
+
+// Device layouts of a tree built on the device back to host records: the 8-bit
+// planes as the host build rounds them, outward from the FP32 ones.
+__global__ void k_unpack_bvh(const DevNodeQ16* __restrict__ nodes, const Bvh8FloatNode* __restrict__ fnodes,
+                             uint32_t n_nodes, const DevTriA* __restrict__ ta, const DevTriB* __restrict__ tb,
+                             uint32_t n_tris, Bvh8Node* __restrict__ out, TriRecord* __restrict__ tris) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_nodes; i += gridDim.x * blockDim.x) {
+        const Bvh8FloatNode s = fnodes[i];
+        Bvh8Node d;
+        d.px = nodes[i].px; d.py = nodes[i].py; d.pz = nodes[i].pz;
+        d.imask = (uint8_t)(s.slots & 0xFFu);
+        d.child_base = s.child_base;
+        d.tri_base = s.tri_base;
+        bool used[8];
+        for (int j = 0; j < 8; ++j) {
+            const uint32_t bits = s.slots >> 8;
+            const uint32_t count = __popc((bits >> (3 * j)) & 7u), below = __popc(bits & ((1u << (3 * j)) - 1u));
+            d.meta[j] = (d.imask >> j) & 1 ? 0x80 : count ? (uint8_t)((count << 5) | below) : 0;
+            used[j] = d.meta[j] != 0;
+        }
+        const float p[3] = {d.px, d.py, d.pz};
+        uint8_t e[3];
+        for (int k = 0; k < 3; ++k) {
+            float top = -FLT_MAX;
+            for (int j = 0; j < 8; ++j)
+                if (used[j]) top = fmaxf(top, s.planes[k][1][j]);
+            const int ek = scale_exponent_d((double)top - (double)p[k]);
+            e[k] = (uint8_t)(ek + 127);
+            const double step = ldexp(1.0, ek);
+            for (int j = 0; j < 8; ++j) {
+                const double lo = floor(((double)s.planes[k][0][j] - (double)p[k]) / step);
+                const double hi = ceil(((double)s.planes[k][1][j] - (double)p[k]) / step);
+                d.qlo[k][j] = used[j] ? (uint8_t)fmax(0.0, fmin(255.0, lo)) : 255;
+                d.qhi[k][j] = used[j] ? (uint8_t)fmax(0.0, fmin(255.0, hi)) : 0;
+            }
+        }
+        d.ex = e[0]; d.ey = e[1]; d.ez = e[2];
+        out[i] = d;
+    }
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_tris; i += gridDim.x * blockDim.x) {
+        const DevTriA a = ta[i];
+        const DevTriB b = tb[i];
+        tris[i] = TriRecord{{a.v1[0], a.v1[1], a.v1[2]}, a.face, {a.e1[0], a.e1[1], a.e1[2]}, 0.f, {a.e2x, b.e2y, b.e2z}, 0.f};
+    }
+}
+
+// Points the scene's device view at its BVH buffers.
+static void view_bvh(crt_scene s, uint32_t n_tris, bool fok) {
+    s->dev.nodes = s->nodes.as<DevNodeQ16>();
+    s->dev.fnodes = fok ? s->fnodes.as<Bvh8FloatNode>() : nullptr;
+    s->dev.tris_a = s->tris.as<DevTriA>();
+    s->dev.tris_b = reinterpret_cast<const DevTriB*>(s->dev.tris_a + n_tris);
+}
+
 // Uploads a built BVH (both node encodings while child indices fit 24 bits)
 // and points the device view and the statistics at it.  The buffers it
 // replaces are freed on return: callers make sure no work still reads them.
@@ -50,20 +148,27 @@ static int install_bvh(crt_scene s, Bvh8& b, uint32_t width) {
     DevBuf nodes, fnodes, tris;
     int st = CRT_OK;
     if (b.fnodes_ok && (st = upload(fnodes, b.fnodes))) return st;
-    if ((st = upload(nodes, b.nodes)) || (st = upload(tris, b.tris))) return st;
+    DevBuf raw_nodes, raw_tris;
+    if ((st = upload(raw_nodes, b.nodes)) || (st = upload(raw_tris, b.tris))) return st;
+    const uint32_t nn = (uint32_t)b.nodes.size(), nt = (uint32_t)b.tris.size();
+    CRT_CUDA(nodes.alloc((size_t)nn * sizeof(DevNodeQ16)));
+    CRT_CUDA(tris.alloc((size_t)nt * (sizeof(DevTriA) + sizeof(DevTriB))));
+    k_pack_bvh<<<(uint32_t)std::min<uint64_t>(((uint64_t)std::max(nn, nt) + 255) / 256, 4096), 256>>>(
+        raw_nodes.as<Bvh8Node>(), b.fnodes_ok ? fnodes.as<Bvh8FloatNode>() : nullptr, nn, raw_tris.as<TriRecord>(), nt, nodes.as<DevNodeQ16>(), tris.as<DevTriA>(),
+        reinterpret_cast<DevTriB*>(tris.as<DevTriA>() + nt));
+    CRT_CUDA(cudaGetLastError());
+    CRT_CUDA(cudaDeviceSynchronize());
     s->nodes.swap(nodes);
     s->fnodes.swap(fnodes);
     s->tris.swap(tris);
     s->bvh = std::move(b);
-    s->dev.nodes = s->nodes.as<float4>();
-    s->dev.fnodes = s->bvh.fnodes_ok ? s->fnodes.as<float4>() : nullptr;
-    s->dev.tris = s->tris.as<float4>();
+    view_bvh(s, nt, s->bvh.fnodes_ok);
     crt_scene_info& I = s->info;
     I.num_nodes = (uint32_t)s->bvh.nodes.size();
     I.max_depth = s->bvh.max_depth;
     I.node_bytes = s->default_f32 ? s->bvh.fnodes.size() * sizeof(Bvh8FloatNode)
-                                  : s->bvh.nodes.size() * sizeof(Bvh8Node);
-    I.triangle_bytes = s->bvh.tris.size() * sizeof(TriRecord);
+                                  : s->bvh.nodes.size() * sizeof(DevNodeQ16);
+    I.triangle_bytes = s->bvh.tris.size() * (sizeof(DevTriA) + sizeof(DevTriB));
     I.bvh_width = width;
     ++s->generation;
     return CRT_OK;
@@ -74,14 +179,17 @@ static int install_bvh(crt_scene s, Bvh8& b, uint32_t width) {
 static int ensure_host_bvh(crt_scene s) {
     if (s->host_bvh) return CRT_OK;
     Bvh8& b = s->bvh;
-    b.nodes.resize(s->info.num_nodes);
-    b.tris.resize(s->info.num_triangles);
-    b.fnodes.resize(b.fnodes_ok ? s->info.num_nodes : 0);
-    CRT_CUDA(cudaMemcpy(b.nodes.data(), s->nodes.p, b.nodes.size() * sizeof(Bvh8Node), cudaMemcpyDeviceToHost));
-    CRT_CUDA(cudaMemcpy(b.tris.data(), s->tris.p, b.tris.size() * sizeof(TriRecord), cudaMemcpyDeviceToHost));
-    if (b.fnodes_ok)
-        CRT_CUDA(cudaMemcpy(b.fnodes.data(), s->fnodes.p, b.fnodes.size() * sizeof(Bvh8FloatNode),
-                            cudaMemcpyDeviceToHost));
+    const uint32_t nn = s->info.num_nodes, nt = s->info.num_triangles;
+    DevBuf raw_nodes, raw_tris;
+    CRT_CUDA(raw_nodes.alloc((size_t)nn * sizeof(Bvh8Node)));
+    CRT_CUDA(raw_tris.alloc((size_t)nt * sizeof(TriRecord)));
+    k_unpack_bvh<<<(uint32_t)std::min<uint64_t>(((uint64_t)std::max(nn, nt) + 255) / 256, 4096), 256>>>(
+        s->dev.nodes, s->fnodes.as<Bvh8FloatNode>(), nn, s->dev.tris_a, s->dev.tris_b, nt, raw_nodes.as<Bvh8Node>(), raw_tris.as<TriRecord>());
+    CRT_CUDA(cudaGetLastError());
+    b.nodes.resize(nn);
+    b.tris.resize(nt);
+    CRT_CUDA(cudaMemcpy(b.nodes.data(), raw_nodes.p, b.nodes.size() * sizeof(Bvh8Node), cudaMemcpyDeviceToHost));
+    CRT_CUDA(cudaMemcpy(b.tris.data(), raw_tris.p, b.tris.size() * sizeof(TriRecord), cudaMemcpyDeviceToHost));
     s->host_bvh = true;
     return CRT_OK;
 }
@@ -105,14 +213,12 @@ static int build_on_device(crt_scene s, const float* dv1, const float* de1, cons
     s->bvh.fnodes_ok = fok;
     s->bvh.max_depth = depth;
     s->host_bvh = false;
-    s->dev.nodes = s->nodes.as<float4>();
-    s->dev.fnodes = fok ? s->fnodes.as<float4>() : nullptr;
-    s->dev.tris = s->tris.as<float4>();
+    view_bvh(s, n, fok);
     crt_scene_info& I = s->info;
     I.num_nodes = nn;
     I.max_depth = depth;
-    I.node_bytes = (size_t)nn * (s->default_f32 ? sizeof(Bvh8FloatNode) : sizeof(Bvh8Node));
-    I.triangle_bytes = (size_t)n * sizeof(TriRecord);
+    I.node_bytes = (size_t)nn * (s->default_f32 ? sizeof(Bvh8FloatNode) : sizeof(DevNodeQ16));
+    I.triangle_bytes = (size_t)n * (sizeof(DevTriA) + sizeof(DevTriB));
     I.bvh_width = width;
     ++s->generation;
     return CRT_OK;

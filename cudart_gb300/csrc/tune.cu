@@ -5,8 +5,8 @@
 // thread per pixel, renderer.cu:543-551) and has nothing to tune.  Here the
 // options that change speed but never the image -- node encoding, traversal
 // block size, shared-memory stack depth, queue entries claimed per fetch,
-// wave sets in flight, paths per wave, lane refill and its threshold, top BVH
-// nodes staged in shared memory, and the BVH's width --
+// wave sets in flight, paths per wave, lane refill and its threshold, and the
+// BVH's width --
 // are searched by coordinate descent: each axis in turn is swept with the
 // others held, and a value is adopted when it beats the current best by more
 // than the noise margin.  Every candidate renders the same samples (a fresh
@@ -117,7 +117,6 @@ struct Tuner {
             {&crt_render_options::wave_sets, {1, 2, 3, 4}},
             {&crt_render_options::wave_paths, {1u << 21, 1u << 22, 1u << 23, 1u << 24, 1u << 25}},
             {&crt_render_options::queue_chunk, {32, 64, 128}},
-            {&crt_render_options::top_nodes, {0, 9, 73}},
         };
         for (const Axis& a : axes) {
             for (uint32_t v : a.values) {

@@ -36,15 +36,13 @@ RenderParams make_params(crt_render r, uint32_t view, uint32_t spp0, uint32_t ns
 
 constexpr int kWaveBlock = 128;            // generate / shade / counting kernels
 constexpr int kTraversalBlockMax = 256;    // extend / shadow: block size chosen at launch
-// Register cap of the traversal kernels: fewer registers, more resident
-// warps to hide the dependent node loads (measured: 56 beats 64, 48 and 40).
+// Register cap of the traversal kernels, both node encodings.  The quantised
+// test needs 61-63 (no spills, 32 warps per SM), the FP32 one spills 28-40 bytes
+// of rarely used state.  Measured on the 1080p frame and the 1001x563 mixed
+// scene: FP32 nodes 56 / 64 / 72 / 80 registers 408 / 380 / 389 / 408 ms, quantised
+// 48 / 56 / 64 / 72 registers 43.0 / 39.6 / 39.5 / 41.0 ms.
 #ifndef CRT_TRAVERSAL_REGS
-#define CRT_TRAVERSAL_REGS 56
-#endif
-// FP32 planes: 56 as well since the window sort (+0.6% on the 1080p frame,
-// +1.1% on the mixed scene over 64, 16 bytes of spill; 72 loses 2-3%).
-#ifndef CRT_TRAVERSAL_REGS_F32
-#define CRT_TRAVERSAL_REGS_F32 56
+#define CRT_TRAVERSAL_REGS 64
 #endif
 constexpr uint32_t kDefaultWaveSets = 4;   // measured: 4 x 32M-path sets +1.2% over 3 at 1080p
 constexpr uint32_t kMaxWaves = 1u << 16;   // descriptors uploaded per chunk
@@ -64,9 +62,8 @@ enum Counter : uint32_t {
 };
 
 // Profiling totals: extension rays, nodes, triangles; shadow rays, nodes, triangles.
-// Visits to the staged top nodes: P_EXT_TOP, P_SHD_TOP.
 enum ProfileCounter : uint32_t {
-    P_EXT_RAYS, P_EXT_NODES, P_EXT_TRIS, P_SHD_RAYS, P_SHD_NODES, P_SHD_TRIS, P_EXT_TOP, P_SHD_TOP, P_COUNT
+    P_EXT_RAYS, P_EXT_NODES, P_EXT_TRIS, P_SHD_RAYS, P_SHD_NODES, P_SHD_TRIS, P_COUNT
 };
 
 // Pixels [p0, p1) x samples [s0, s1) of view `view`: path slot0 +
@@ -149,7 +146,6 @@ struct WaveParams {
     unsigned long long* prof;   // ProfileCounter totals (profiling pass only)
     int stack_depth;            // traversal stack entries in shared memory
     uint32_t queue_chunk;       // queue entries a warp claims per fetch (batch mode)
-    uint32_t top_nodes;         // BVH nodes staged in shared memory by extend / shadow
     uint32_t refill_busy;       // lane refill: busy lanes at or below which idle lanes refill
     // adjoint replay only
     const float4* adj;          // d(objective)/d(radiance sum), per pixel of every view
@@ -470,23 +466,13 @@ struct ExtendJob {
     }
 };
 
-// Copies the first W.top_nodes nodes to the start of dynamic shared memory
-// and returns where the stacks begin (TOP = false: no staging at all).
-template <bool F32, bool TOP>
-CRT_D uint2* stage_top_nodes(const WaveParams& W) {
-    if (!TOP) return reinterpret_cast<uint2*>(crt_top_nodes);
-    const uint32_t n = W.top_nodes * (F32 ? 13u : 5u);
-    const float4* src = F32 ? W.R.S.fnodes : W.R.S.nodes;
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) crt_top_nodes[i] = ldg(src + i);
-    __syncthreads();
-    return reinterpret_cast<uint2*>(crt_top_nodes + n);
-}
+// Dynamic shared memory of the traversal kernels: the stacks.
+extern __shared__ uint2 crt_stacks[];
 
-template <bool REFILL, bool WHOLE_LEAF, bool F32, bool TOP>
-__global__ void __maxnreg__(F32 ? CRT_TRAVERSAL_REGS_F32 : CRT_TRAVERSAL_REGS) wf_extend(WaveParams W) {
-    uint2* stacks = stage_top_nodes<F32, TOP>(W);
+template <bool REFILL, bool WHOLE_LEAF, bool F32>
+__global__ void __maxnreg__(CRT_TRAVERSAL_REGS) wf_extend(WaveParams W) {
     StackSpill overflow;
-    Stack st(stacks, overflow, blockDim.x, W.stack_depth, TOP ? W.top_nodes : 0u);
+    Stack st(crt_stacks, overflow, blockDim.x, W.stack_depth);
     const uint32_t cur = W.counters[C_CUR];
     __shared__ uint32_t pre_sh[9];
     ExtendJob<WHOLE_LEAF, F32> job(W, queue_view(W, cur, pre_sh), st);
@@ -762,23 +748,21 @@ struct ShadowJob {
 // and a visible light adds d objective / d (light material ka).  Dynamic
 // shared memory: the traversal stacks, then [n_mats][6] gradient floats.
 template <bool F32>
-__global__ void __maxnreg__(F32 ? CRT_TRAVERSAL_REGS_F32 : CRT_TRAVERSAL_REGS) wf_shadow_adj(WaveParams W) {
-    uint2* stacks = stage_top_nodes<F32, true>(W);
-    float* grad = reinterpret_cast<float*>(stacks + (size_t)blockDim.x * W.stack_depth);
+__global__ void __maxnreg__(CRT_TRAVERSAL_REGS) wf_shadow_adj(WaveParams W) {
+    float* grad = reinterpret_cast<float*>(crt_stacks + (size_t)blockDim.x * W.stack_depth);
     zero_grad_block(grad, W.n_mats);
     StackSpill overflow;
-    Stack st(stacks, overflow, blockDim.x, W.stack_depth, W.top_nodes);
+    Stack st(crt_stacks, overflow, blockDim.x, W.stack_depth);
     ShadowJob<true, F32, true> job(W, st, grad);
     persistent_loop<false>(W.counters[C_SHADOW], &W.counters[C_FETCH_SHD], W.queue_chunk, 31u, job);
     count_rays(W.R.ray_counts, 0, job.rays);
     flush_grad_block(W, grad);
 }
 
-template <bool REFILL, bool WHOLE_LEAF, bool F32, bool TOP>
-__global__ void __maxnreg__(F32 ? CRT_TRAVERSAL_REGS_F32 : CRT_TRAVERSAL_REGS) wf_shadow(WaveParams W) {
-    uint2* stacks = stage_top_nodes<F32, TOP>(W);
+template <bool REFILL, bool WHOLE_LEAF, bool F32>
+__global__ void __maxnreg__(CRT_TRAVERSAL_REGS) wf_shadow(WaveParams W) {
     StackSpill overflow;
-    Stack st(stacks, overflow, blockDim.x, W.stack_depth, TOP ? W.top_nodes : 0u);
+    Stack st(crt_stacks, overflow, blockDim.x, W.stack_depth);
     ShadowJob<WHOLE_LEAF, F32> job(W, st);
     persistent_loop<REFILL>(W.counters[C_SHADOW], &W.counters[C_FETCH_SHD], W.queue_chunk, W.refill_busy, job);
     count_rays(W.R.ray_counts, 0, job.rays);
@@ -786,30 +770,28 @@ __global__ void __maxnreg__(F32 ? CRT_TRAVERSAL_REGS_F32 : CRT_TRAVERSAL_REGS) w
 
 using WaveKernel = void (*)(WaveParams);
 
-// Kernel variants by the CRT_FLAG_* traversal-scheduling flags, the node
-// format and whether top nodes are staged in shared memory.
-template <bool F32, bool TOP>
+// Kernel variants by the CRT_FLAG_* traversal-scheduling flags and the node
+// format.
+template <bool F32>
 static WaveKernel extend_kernel_f(uint32_t flags) {
     const bool refill = flags & CRT_FLAG_LANE_REFILL, whole = !(flags & CRT_FLAG_SPLIT_LEAF);
-    if (refill) return whole ? wf_extend<true, true, F32, TOP> : wf_extend<true, false, F32, TOP>;
-    return whole ? wf_extend<false, true, F32, TOP> : wf_extend<false, false, F32, TOP>;
+    if (refill) return whole ? wf_extend<true, true, F32> : wf_extend<true, false, F32>;
+    return whole ? wf_extend<false, true, F32> : wf_extend<false, false, F32>;
 }
 
-template <bool F32, bool TOP>
+template <bool F32>
 static WaveKernel shadow_kernel_f(uint32_t flags) {
     const bool refill = flags & CRT_FLAG_LANE_REFILL, whole = !(flags & CRT_FLAG_SPLIT_LEAF);
-    if (refill) return whole ? wf_shadow<true, true, F32, TOP> : wf_shadow<true, false, F32, TOP>;
-    return whole ? wf_shadow<false, true, F32, TOP> : wf_shadow<false, false, F32, TOP>;
+    if (refill) return whole ? wf_shadow<true, true, F32> : wf_shadow<true, false, F32>;
+    return whole ? wf_shadow<false, true, F32> : wf_shadow<false, false, F32>;
 }
 
-static WaveKernel extend_kernel(uint32_t flags, bool f32, bool top) {
-    if (f32) return top ? extend_kernel_f<true, true>(flags) : extend_kernel_f<true, false>(flags);
-    return top ? extend_kernel_f<false, true>(flags) : extend_kernel_f<false, false>(flags);
+static WaveKernel extend_kernel(uint32_t flags, bool f32) {
+    return f32 ? extend_kernel_f<true>(flags) : extend_kernel_f<false>(flags);
 }
 
-static WaveKernel shadow_kernel(uint32_t flags, bool f32, bool top) {
-    if (f32) return top ? shadow_kernel_f<true, true>(flags) : shadow_kernel_f<true, false>(flags);
-    return top ? shadow_kernel_f<false, true>(flags) : shadow_kernel_f<false, false>(flags);
+static WaveKernel shadow_kernel(uint32_t flags, bool f32) {
+    return f32 ? shadow_kernel_f<true>(flags) : shadow_kernel_f<false>(flags);
 }
 
 __global__ void wf_flip(WaveParams W) {
@@ -885,11 +867,6 @@ CRT_D void add_profile(unsigned long long* p, uint32_t rays, uint32_t nodes, uin
     }
 }
 
-CRT_D void add_top(unsigned long long* p, uint32_t top) {
-    const uint32_t t = __reduce_add_sync(0xFFFFFFFFu, top);
-    if ((threadIdx.x & 31u) == 0 && t) atomicAdd(p, (unsigned long long)t);
-}
-
 // Counting re-runs (profiling only): the same traversals as wf_extend /
 // wf_shadow over the same queue entries, tallying node visits and triangle
 // tests instead of writing results.
@@ -904,7 +881,7 @@ __global__ void __launch_bounds__(kWaveBlock) wf_extend_count(WaveParams W) {
     const QueueView q = queue_view(W, cur, pre_sh);
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t rays = 0;
-    TraversalStats ts{0, 0, 0, W.top_nodes};
+    TraversalStats ts{0, 0};
     for (;;) {
         uint32_t base = 0;
         if (lane == 0) base = atomicAdd(&W.counters[C_FETCH_CNT], 32u);
@@ -924,7 +901,6 @@ __global__ void __launch_bounds__(kWaveBlock) wf_extend_count(WaveParams W) {
         }
     }
     add_profile(W.prof + P_EXT_RAYS, rays, ts.nodes, ts.tris);
-    add_top(W.prof + P_EXT_TOP, ts.top);
 }
 
 template <bool F32>
@@ -935,7 +911,7 @@ __global__ void __launch_bounds__(kWaveBlock) wf_shadow_count(WaveParams W) {
     const uint32_t n = W.counters[C_SHADOW];
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t rays = 0;
-    TraversalStats ts{0, 0, 0, W.top_nodes};
+    TraversalStats ts{0, 0};
     for (;;) {
         uint32_t base = 0;
         if (lane == 0) base = atomicAdd(&W.counters[C_FETCH_CNT], 32u);
@@ -954,7 +930,6 @@ __global__ void __launch_bounds__(kWaveBlock) wf_shadow_count(WaveParams W) {
         }
     }
     add_profile(W.prof + P_SHD_RAYS, rays, ts.nodes, ts.tris);
-    add_top(W.prof + P_SHD_TOP, ts.top);
 }
 
 int persistent_grid(const void* kernel, int block, size_t smem) {
@@ -1106,7 +1081,6 @@ static WaveParams wave_params(crt_render r, WaveSet& set) {
     W.prof = B.prof.as<unsigned long long>();
     W.stack_depth = (int)traversal_stack(r->opts);
     W.queue_chunk = queue_chunk(r->opts);
-    W.top_nodes = staged_nodes(r->scene, r->opts);
     W.refill_busy = refill_busy(r->opts);
     W.octant = B.octant;
     W.shadow_q = window_sort(r->opts.flags) ? B.shadow_q.as<uint32_t>() : nullptr;
@@ -1124,18 +1098,17 @@ struct WaveGrids {
 
 
 // Kernel choice and launch shapes, queried before a capture starts.
-static WaveGrids wave_grids(uint32_t capacity, uint32_t flags, bool f32, uint32_t block, uint32_t depth,
-                            uint32_t top_nodes) {
+static WaveGrids wave_grids(uint32_t capacity, uint32_t flags, bool f32, uint32_t block, uint32_t depth) {
     WaveGrids g;
-    g.extend = extend_kernel(flags, f32, top_nodes > 0);
-    g.shadow = shadow_kernel(flags, f32, top_nodes > 0);
+    g.extend = extend_kernel(flags, f32);
+    g.shadow = shadow_kernel(flags, f32);
     g.extend_count = f32 ? wf_extend_count<true> : wf_extend_count<false>;
     g.shadow_count = f32 ? wf_shadow_count<true> : wf_shadow_count<false>;
     const bool sort = window_sort(flags);
     g.shade = sort ? wf_shade<false, true> : wf_shade<false, false>;
     g.shade_adj = sort ? wf_shade<true, true> : wf_shade<true, false>;
     g.tblock = (int)block;
-    g.tsmem = (size_t)top_nodes * (f32 ? sizeof(Bvh8FloatNode) : sizeof(Bvh8Node)) + (size_t)block * depth * sizeof(uint2);
+    g.tsmem = (size_t)block * depth * sizeof(uint2);
     cudaFuncSetAttribute((const void*)g.extend, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.tsmem);
     cudaFuncSetAttribute((const void*)g.shadow, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.tsmem);
     g.gen = grid_for(capacity, kWaveBlock, 16);
@@ -1147,8 +1120,7 @@ static WaveGrids wave_grids(uint32_t capacity, uint32_t flags, bool f32, uint32_
 }
 
 static WaveGrids wave_grids(crt_render r, uint32_t capacity) {
-    return wave_grids(capacity, r->opts.flags, uses_f32_nodes(r), traversal_block(r->opts), traversal_stack(r->opts),
-                      staged_nodes(r->scene, r->opts));
+    return wave_grids(capacity, r->opts.flags, uses_f32_nodes(r), traversal_block(r->opts), traversal_stack(r->opts));
 }
 
 // Enqueue the body of one wave (generation and every bounce); captured into
@@ -1654,8 +1626,6 @@ int wavefront_profile_pass(crt_render r, const std::vector<ViewWork>& work, crt_
     out->shadow_rays += c[P_SHD_RAYS];
     out->shadow_nodes += c[P_SHD_NODES];
     out->shadow_tris += c[P_SHD_TRIS];
-    out->extension_top_nodes += c[P_EXT_TOP];
-    out->shadow_top_nodes += c[P_SHD_TOP];
     return CRT_OK;
 }
 
@@ -1790,11 +1760,10 @@ extern "C" int crt_render_tile_noalloc(crt_scene scene, const crt_camera* camera
     W.prof = nullptr;
     W.stack_depth = (int)traversal_stack(o);
     W.queue_chunk = queue_chunk(o);
-    W.top_nodes = staged_nodes(scene, o);
     W.refill_busy = refill_busy(o);
     W.octant = false;   // the scratch holds single-region queues
     W.capacity = kNoAllocPaths;
-    const WaveGrids G = wave_grids(kNoAllocPaths, o.flags, f32, traversal_block(o), W.stack_depth, W.top_nodes);
+    const WaveGrids G = wave_grids(kNoAllocPaths, o.flags, f32, traversal_block(o), W.stack_depth);
     cudaStream_t s = (cudaStream_t)stream;
     DevView view;
     view.cam = R.cam;

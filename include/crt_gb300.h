@@ -139,12 +139,12 @@ typedef enum {
                             millions of triangles */
 } crt_bvh_builder;
 
-/* BVH node encoding on the device (same tree either way). */
+/* BVH node encoding on the device (same tree, same results either way). */
 typedef enum {
-    CRT_NODES_Q8 = 0,    /* 80-byte nodes, child planes quantised to 8 bits
-                            relative to the node and rounded outward */
-    CRT_NODES_F32 = 1    /* 208-byte nodes with FP32 child planes: more bytes
-                            per visit, half the ALU work per child test */
+    CRT_NODES_Q8 = 0,    /* quantised nodes: child planes as 16-bit floats relative to
+                            the node, rounded outward; 160 bytes apart, 120 read.  The
+                            faster one on every workload measured */
+    CRT_NODES_F32 = 1    /* 208-byte nodes with FP32 child planes */
 } crt_node_format;
 
 typedef struct crt_scene_s* crt_scene;
@@ -153,13 +153,13 @@ typedef struct crt_render_s* crt_render;
 /* Build-time statistics of a scene's BVH and buffers. */
 typedef struct {
     uint32_t num_triangles;
-    uint32_t num_nodes;        /* 8-wide nodes (80 bytes each) */
+    uint32_t num_nodes;        /* 8-wide nodes */
     uint32_t max_depth;        /* levels from the root to the deepest leaf */
     uint32_t num_lights;
     uint32_t num_materials;
     uint32_t num_textures;
     uint64_t node_bytes;
-    uint64_t triangle_bytes;   /* intersection records (48 bytes each) */
+    uint64_t triangle_bytes;   /* intersection records (40 bytes each) */
     uint64_t shading_bytes;    /* normals/uv/material records */
     uint64_t texture_bytes;
     float lights_area;
@@ -187,7 +187,7 @@ CRT_EXPORT int crt_camera_from_json(float fov_deg, float focal_length, float fst
 CRT_EXPORT int crt_scene_create(const crt_scene_desc* desc, crt_scene* out);
 CRT_EXPORT int crt_scene_destroy(crt_scene scene);
 CRT_EXPORT int crt_scene_get_info(crt_scene scene, crt_scene_info* out);
-/* Host copies of the BVH as uploaded: nodes [num_nodes][80 bytes],
+/* Host copies of the BVH: nodes [num_nodes][80 bytes, child planes in 8 bits],
  * triangle records [num_triangles][48 bytes] (v1.xyz + face index bits,
  * e1.xyz + 0, e2.xyz + 0).  Either pointer may be NULL. */
 CRT_EXPORT int crt_scene_export_bvh(crt_scene scene, void* nodes, void* triangles);
@@ -320,11 +320,9 @@ typedef struct {
     uint32_t queue_chunk;      /* wavefront traversal kernels: queue entries a warp
                                   claims per fetch, 32, 64, 128 or 256 (0 = 32);
                                   unused with CRT_FLAG_LANE_REFILL */
-    uint32_t top_nodes;        /* wavefront traversal kernels: the first top_nodes
-                                  BVH nodes (breadth-first: the top levels) are
-                                  copied to shared memory at kernel start, 0..128
-                                  (0 = none; 9 = two levels, the default of
-                                  crt_render_options_default; 73 = three) */
+    uint32_t top_nodes;        /* 0..128; without effect.  It once staged the tree's top
+                                  nodes in shared memory; since the nodes lie spread over
+                                  the L1 banks, reading them there is faster */
     uint32_t refill_busy;      /* with CRT_FLAG_LANE_REFILL: idle lanes of a warp
                                   take new rays together once at most this many
                                   lanes are still busy, 1..31 (0 = 31: as soon as
@@ -389,8 +387,8 @@ typedef struct {
     uint64_t extend_rays_by_bounce[16];
     double shadow_ms_by_bounce[16];
     uint64_t shadow_rays_by_bounce[16];
-    uint64_t extension_top_nodes, shadow_top_nodes;   /* visits (in *_nodes) to the nodes
-                                                         staged in shared memory (top_nodes) */
+    uint64_t extension_top_nodes, shadow_top_nodes;   /* always 0: no node is read from
+                                                         shared memory */
 } crt_stage_profile;
 
 /* Renders n_spp more samples per pixel (like crt_render_pass, same result)
@@ -510,7 +508,7 @@ CRT_EXPORT int crt_render_ray_counts(crt_render r, uint64_t* extension_rays, uin
  * short wavefront renders of the given scene, camera and image size and
  * searches, by coordinate descent, the options that change speed but not
  * the image: node_format, block_size, stack_depth, queue_chunk, wave_sets,
- * wave_paths, CRT_FLAG_LANE_REFILL, top_nodes and (tune_bvh_width) the BVH
+ * wave_paths, CRT_FLAG_LANE_REFILL and (tune_bvh_width) the BVH
  * width.
  * The device must be otherwise idle for the timings to mean anything.  With
  * tune_bvh_width the scene's BVH is rebuilt (crt_scene_set_bvh_width) and
