@@ -18,21 +18,27 @@ int wavefront_adjoint(crt_render r, const std::vector<ViewWork>& work, const flo
                       uint32_t flags);
 
 constexpr int kMegaBlock = 128;         // 16 x 8 pixel tile, warps of 8 x 4
-constexpr uint32_t kMegaSppPerLaunch = 4;
+constexpr int kMegaStack = 8;           // stack entries per thread in shared memory
+constexpr uint32_t kMegaSppPerLaunch = 16;
 
 // One thread per pixel; samples [spp0, spp0 + nspp) are added to the FP32
 // accumulator in sample order, so the sums equal the reference's per-pass
 // accumulation (`p_imgBuffer[idx] += color`, parallel_renderer.cu:340).
+//
+// One turn of the loop is one bounce of whichever sample the lane is at, so a
+// lane whose path ended starts its next sample beside the other lanes' later
+// bounces instead of waiting for the warp's longest path.  Bound by issue slots
+// at half-filled warps.  1280x720 x 16, mixed scene, alone: 56.5 ms with the
+// sample loop outside the bounce loop and 4 samples per launch, 55.9 with this
+// loop and 4, 52.3 with 16.  A resident grid whose lanes go on to further tiles
+// lost 5-20% on scenes larger than L1 (rays of one warp from distant pixels).
+// Register cap, FP32 / quantised nodes on that frame: 80 54.8 / 52.5, 96 52.2 /
+// 52.0, 112 57.6 / - ms.
 template <bool F32>
-// Register cap of the megakernel (the whole path lives in registers):
-// measured 80 best against 64, 96 and the uncapped 128.
-#ifndef CRT_MEGA_REGS
-#define CRT_MEGA_REGS 80
-#endif
-__global__ void __maxnreg__(F32 ? CRT_MEGA_REGS + 16 : CRT_MEGA_REGS) mega_kernel(RenderParams P) {
-    __shared__ uint2 stack_sh[kStackShared * kMegaBlock];
+__global__ void __maxnreg__(96) mega_kernel(RenderParams P) {
+    __shared__ uint2 stack_sh[kMegaStack * kMegaBlock];
     StackSpill overflow;
-    Stack st(stack_sh, overflow, kMegaBlock, kStackShared);
+    Stack st(stack_sh, overflow, kMegaBlock, kMegaStack);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t x = blockIdx.x * 16u + (warp & 1u) * 8u + (lane & 7u);
     const uint32_t y = blockIdx.y * 8u + (warp >> 1) * 4u + (lane >> 3);
@@ -40,11 +46,17 @@ __global__ void __maxnreg__(F32 ? CRT_MEGA_REGS + 16 : CRT_MEGA_REGS) mega_kerne
     if (x < P.width && y < P.height) {
         const uint32_t pixel = y * P.width + x;
         float4 acc = P.accum[pixel];
-        for (uint32_t s = 0; s < P.nspp; ++s) {
-            const float3 c = sample_path<F32>(P, (int)x, (int)y, pixel, P.spp0 + s, st, n_ext, n_shadow);
-            acc.x = acc.x + c.x;
-            acc.y = acc.y + c.y;
-            acc.z = acc.z + c.z;
+        PathState ps;
+        Ray ray;
+        bool alive = false;
+        for (uint32_t s = 0; alive || s < P.nspp;) {
+            if (!alive) begin_path(P.cam, P.seed, P.view, x, y, pixel, P.spp0 + s++, ps, ray);
+            alive = path_bounce<F32>(P, ps, ray, st, n_ext, n_shadow);
+            if (!alive) {
+                acc.x = acc.x + ps.color.x;
+                acc.y = acc.y + ps.color.y;
+                acc.z = acc.z + ps.color.z;
+            }
         }
         P.accum[pixel] = acc;
     }

@@ -195,32 +195,28 @@ CRT_D bool occluded(const DevScene& S, const ShadowReq& sr, Stack& st) {
     return traverse<true, false, F32>(S, sr.o, sr.d, kEps, h, (int32_t)sr.light_face, st, nullptr);
 }
 
+// One bounce of a path: closest hit, shading and the shadow test.  Returns
+// whether the path continues; if not, ps.color is its radiance.
 template <bool F32>
-CRT_D float3 sample_path(const RenderParams& P, int x, int y, uint32_t pixel, uint32_t sample, Stack& st,
-                         uint32_t& n_ext, uint32_t& n_shadow) {
-    PathState ps;
-    Ray ray;
-    begin_path(P.cam, P.seed, P.view, (uint32_t)x, (uint32_t)y, pixel, sample, ps, ray);
-    for (uint32_t bounce = 0; bounce < P.max_depth; ++bounce) {
-        Hit h;
-        h.t = FLT_MAX;
-        h.face = -1;
-        h.u = h.v = 0.f;
-        ++n_ext;
-        traverse<false, false, F32>(P.S, ray.o, ray.d, kEps, h, -1, st, nullptr);
-        if (h.face < 0) {
-            shade_miss(ps);
-            break;
-        }
-        ShadowReq sr;
-        const bool alive = shade_hit(P, ps, ray, h, sr);
-        if (sr.valid) {
-            ++n_shadow;
-            if (!occluded<F32>(P.S, sr, st)) ps.color = ps.color + sr.contrib;
-        }
-        if (!alive) break;
+CRT_D bool path_bounce(const RenderParams& P, PathState& ps, Ray& ray, Stack& st, uint32_t& n_ext,
+                       uint32_t& n_shadow) {
+    Hit h;
+    h.t = FLT_MAX;
+    h.face = -1;
+    h.u = h.v = 0.f;
+    ++n_ext;
+    traverse<false, false, F32>(P.S, ray.o, ray.d, kEps, h, -1, st, nullptr);
+    if (h.face < 0) {
+        shade_miss(ps);
+        return false;
     }
-    return ps.color;
+    ShadowReq sr;
+    const bool alive = shade_hit(P, ps, ray, h, sr) && ps.bounce < P.max_depth;
+    if (sr.valid) {
+        ++n_shadow;
+        if (!occluded<F32>(P.S, sr, st)) ps.color = ps.color + sr.contrib;
+    }
+    return alive;
 }
 
 CRT_D void count_rays(unsigned long long* counts, uint32_t ext, uint32_t shadow) {
