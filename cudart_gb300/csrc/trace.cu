@@ -2,25 +2,34 @@
 // instrumented traversal that counts node visits and triangle tests per ray.
 //
 // Replaces intersectBVH (src/renderer/renderer.cu:283-330) for batches of
-// arbitrary rays.  One thread per ray, 128-thread blocks, grid-stride loop
-// over a grid that is a multiple of the SM count.
+// arbitrary rays.  One thread per ray.
 #include "crt_internal.h"
 
 namespace crt {
 
-constexpr int kTraceBlock = 128;
+// One warp per block and a block per 32 rays: rays of arbitrary batches differ
+// widely in length, and a warp that is done makes room for the next at once (32
+// blocks of 64 registers fill an SM's 32 block slots).  Scattered gathers from L2
+// bound the kernel, so resident warps count most.  8.4M rays into the
+// 2.17M-triangle scene, FP32 / quantised nodes: uncapped registers 5.35 / 4.08
+// ms; 64 registers in 128-thread blocks striding over 16 blocks per SM 4.33 / 3.97,
+// one block per 128 rays 4.33 / 3.92, per 64 4.19 / 3.81, per 32 4.10 / 3.75; 56
+// registers 4.71 / 3.97, 72 5.13 / 4.66.  Stacks of 4 or 16 shared entries: within 1%.
+constexpr int kTraceBlock = 32;
+constexpr int kTraceStack = 8;
 
 template <bool COUNT, bool F32>
-__global__ void __launch_bounds__(kTraceBlock) trace_closest_kernel(DevScene S, const float4* __restrict__ rays,
+__global__ void __maxnreg__(64) trace_closest_kernel(DevScene S, const float4* __restrict__ rays,
                                                                     uint32_t n, int32_t* __restrict__ out_face,
                                                                     float* __restrict__ out_t,
                                                                     float2* __restrict__ out_uv,
                                                                     uint32_t* __restrict__ out_nodes,
                                                                     uint32_t* __restrict__ out_tris) {
-    __shared__ uint2 stack_sh[kStackShared * kTraceBlock];
+    __shared__ uint2 stack_sh[kTraceStack * kTraceBlock];
     StackSpill overflow;
-    Stack st(stack_sh, overflow, kTraceBlock, kStackShared);
-    for (uint32_t i = blockIdx.x * kTraceBlock + threadIdx.x; i < n; i += gridDim.x * kTraceBlock) {
+    Stack st(stack_sh, overflow, kTraceBlock, kTraceStack);
+    const uint32_t i = blockIdx.x * kTraceBlock + threadIdx.x;
+    if (i < n) {
         const float4 a = rays[2ull * i], b = rays[2ull * i + 1];
         Hit h;
         h.t = b.w;
@@ -90,7 +99,7 @@ int crt_trace_closest(crt_scene s, const float* d_rays, uint32_t n, int32_t* d_i
     if (n == 0) return CRT_OK;
     if (((uintptr_t)d_rays & 15u) != 0) return set_error(CRT_ERR_INVALID, "rays must be 16-byte aligned");
     auto k = s->default_f32 ? trace_closest_kernel<false, true> : trace_closest_kernel<false, false>;
-    k<<<grid_for(n, kTraceBlock, 16), kTraceBlock, 0, (cudaStream_t)stream>>>(
+    k<<<(n - 1) / kTraceBlock + 1, kTraceBlock, 0, (cudaStream_t)stream>>>(
         s->view(s->default_f32), (const float4*)d_rays, n, d_index, d_t, (float2*)d_uv, nullptr, nullptr);
     CRT_CUDA(cudaGetLastError());
     return CRT_OK;
@@ -103,7 +112,7 @@ int crt_trace_counts(crt_scene s, const float* d_rays, uint32_t n, uint32_t* d_n
     if (n == 0) return CRT_OK;
     if (((uintptr_t)d_rays & 15u) != 0) return set_error(CRT_ERR_INVALID, "rays must be 16-byte aligned");
     auto k = s->default_f32 ? trace_closest_kernel<true, true> : trace_closest_kernel<true, false>;
-    k<<<grid_for(n, kTraceBlock, 16), kTraceBlock, 0, (cudaStream_t)stream>>>(
+    k<<<(n - 1) / kTraceBlock + 1, kTraceBlock, 0, (cudaStream_t)stream>>>(
         s->view(s->default_f32), (const float4*)d_rays, n, nullptr, nullptr, nullptr, d_nodes, d_tris);
     CRT_CUDA(cudaGetLastError());
     return CRT_OK;
