@@ -121,6 +121,7 @@ struct crt_render_s {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     crt::DevBuf accum, lut, ray_counts, view_table, staging;
+    crt::DevBuf path_color;         // radiance per path of a pass on the path kernel
     std::vector<WaveSet> sets;
     uint32_t scene_generation = 0;  // scene BVH the captured wave graphs point at
     cudaEvent_t pass_start = nullptr;

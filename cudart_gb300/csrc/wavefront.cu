@@ -1337,12 +1337,100 @@ static int build_pass_graph(crt_render r, size_t n_waves, uint32_t K) {
     return CRT_OK;
 }
 
+// A few paths, each from its camera ray to its end in one thread, and a second
+// kernel that adds them up pixel by pixel in sample order: two dependent
+// launches instead of four per bounce, and no bounce waits for the slowest ray
+// of all paths.  What bounds it is the latency of one warp's serial visits, so
+// while the chip has warps to spare a warp holds fewer paths and diverges less
+// (`lanes` of the 32 carry one).
+constexpr int kPathStack = 8;   // stack entries per thread in shared memory
+
+template <bool F32>
+__global__ void __maxnreg__(96) path_kernel(RenderParams P, uint32_t pixel0, uint32_t n, uint32_t lanes,
+                                            float4* __restrict__ color) {
+    __shared__ uint2 stack_sh[kPathStack * 32];
+    StackSpill overflow;
+    Stack st(stack_sh, overflow, 32, kPathStack);
+    const uint32_t i = blockIdx.x * lanes + threadIdx.x;
+    uint32_t n_ext = 0, n_shadow = 0;
+    if (threadIdx.x < lanes && i < n) {
+        const uint32_t k = i / P.nspp, pixel = pixel0 + k;
+        PathState ps;
+        Ray ray;
+        begin_path(P.cam, P.seed, P.view, pixel % P.width, pixel / P.width, pixel, P.spp0 + (i - k * P.nspp), ps, ray);
+        while (path_bounce<F32>(P, ps, ray, st, n_ext, n_shadow)) {
+        }
+        color[i] = make_float4(ps.color.x, ps.color.y, ps.color.z, 0.f);
+    }
+    count_rays(P.ray_counts, n_ext, n_shadow);
+}
+
+__global__ void path_sum_kernel(RenderParams P, uint32_t pixel0, uint32_t pixels, const float4* __restrict__ color) {
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= pixels) return;
+    float4 acc = P.accum[pixel0 + k];
+    for (uint32_t s = 0; s < P.nspp; ++s) {
+        const float4 c = color[(size_t)k * P.nspp + s];
+        acc.x = acc.x + c.x;
+        acc.y = acc.y + c.y;
+        acc.z = acc.z + c.z;
+    }
+    P.accum[pixel0 + k] = acc;
+}
+
+// Queues samples [P.spp0, P.spp0 + P.nspp) of pixels [pixel0, pixel0 + pixels):
+// pixels * nspp paths; `color` holds one float4 per path.
+//
+// Paths per warp: as few as keep the warps near what the chip holds at once
+// (20 per SM at 96 registers, 3,040), which halves the divergence a warp pays
+// for.  Measured with 32 / 16 / 8 / 4 / 2 / 1 paths per warp, mixed scene, us: 65,536
+// paths 519 / 426 / 471 / 533 / 683 / 877, 16,384 paths 414 / 331 / 294 / 234 / 263 /
+// 275, 2,048 paths 383 / 323 / 245 / 190 / 154 / 126.
+static void launch_paths(const RenderParams& P, bool f32, uint32_t pixel0, uint32_t pixels, float4* color,
+                         cudaStream_t s) {
+    static const int room[2] = {persistent_grid((const void*)path_kernel<false>, 32, 0),
+                                persistent_grid((const void*)path_kernel<true>, 32, 0)};
+    const uint32_t n = pixels * P.nspp, most = (uint32_t)room[f32] * 11u / 8u;
+    uint32_t lanes = 32;
+    while (lanes > 1 && (n - 1) / (lanes / 2) + 1 <= most) lanes /= 2;
+    (f32 ? path_kernel<true> : path_kernel<false>)<<<(n - 1) / lanes + 1, 32, 0, s>>>(P, pixel0, n, lanes, color);
+    path_sum_kernel<<<(pixels - 1) / 256 + 1, 256, 0, s>>>(P, pixel0, pixels, color);
+}
+
+// Passes of at most this many paths run on the path kernel.  Wave / path kernel
+// at 65,536 paths: mixed scene 0.96 / 0.63 ms, 2.17M triangles 1.05 / 0.38, Cornell
+// box 0.37 / 0.19; at 262,144: 1.21 / 1.39, 1.45 / 0.74, 0.44 / 0.34.  (And no path
+// state is allocated: a first pass of the wave form allocates gigabytes.)
+constexpr uint64_t kDirectPaths = 1u << 17;
+
+// Whether a pass takes the path kernel: a single view, few paths, and no launch
+// shape asked for (an explicit wave size, set count, block size and so on is the
+// caller's choice of the wavefront form).
+static bool direct_pass(crt_render r, const std::vector<ViewWork>& work) {
+    const crt_render_options& o = r->opts;
+    if (work.size() != 1 || o.wave_paths || o.wave_sets || o.flags || o.block_size || o.stack_depth || o.queue_chunk)
+        return false;
+    return (uint64_t)r->views[0].npix() * work[0].nspp <= kDirectPaths;
+}
+
 // A pass: wave w runs on set w % K.  Each set's stream replays its graph for
 // the wave body, then waits for the previous wave's accumulate (on whichever
 // set ran it) before accumulating, so every pixel adds its samples in sample
 // order while the bodies of consecutive waves overlap: one wave's thin late
 // bounces share the GPU with the next wave's heavy first bounces.
 int wavefront_pass(crt_render r, const std::vector<ViewWork>& work) {
+    if (direct_pass(r, work)) {
+        const uint32_t npix = r->views[0].npix();
+        const size_t bytes = (size_t)npix * work[0].nspp * sizeof(float4);
+        if (r->path_color.bytes < bytes) {
+            CRT_CUDA(cudaStreamSynchronize(r->stream));
+            CRT_CUDA(r->path_color.alloc(bytes));
+        }
+        launch_paths(make_params(r, 0, work[0].spp0, work[0].nspp), uses_f32_nodes(r), 0, npix,
+                     r->path_color.as<float4>(), r->stream);
+        CRT_CUDA(cudaGetLastError());
+        return CRT_OK;
+    }
     const uint32_t K = r->opts.wave_sets ? r->opts.wave_sets : kDefaultWaveSets;
     int st = ensure_wave_sets(r, K);
     if (st != CRT_OK) return st;
@@ -1637,32 +1725,19 @@ int wavefront_profile_pass(crt_render r, const std::vector<ViewWork>& work, crt_
 // application that owns every device allocation through its own pool (a
 // plugin inside a DCC tool or game engine), or a latency-sensitive loop that
 // must not pay for cudaMalloc / cudaFree and the synchronisation they imply.
-// For them the wavefront kernels can run on a fixed scratch area that lives
-// in this file as a static device array: every GPU that loads the library
-// holds kNoAllocBytes (about 8.5 MiB) of it until the process exits.  The
-// caller brings the inputs (a scene) and the output (an accumulator); the
-// paths in flight, queues, counters and the wave descriptor use the scratch.
+// For them the path kernel runs on a fixed scratch area that lives in this
+// file as a static device array: every GPU that loads the library holds 1 MiB of
+// it until the process exits.  The caller brings the inputs (a scene) and the
+// output (an accumulator); the scratch holds each path's radiance.
+//
+// The wavefront form's four launches per bounce cost a 64K-path tile 918 us
+// (mixed scene, depth 8; 1,104 us before the node layouts): every bounce waited
+// for its slowest ray.  The path kernel takes 415 us.
 // ---------------------------------------------------------------------------
 Camera to_device_camera(const crt_camera& c);
 
 constexpr uint32_t kNoAllocPaths = CRT_NOALLOC_MAX_PATHS;
-constexpr size_t kNoAllocOff[] = {
-    0,                                  // o | d pairs   32 B per path (two slices)
-    16ull * kNoAllocPaths,
-    32ull * kNoAllocPaths,              // color | mask pairs   32 B per path
-    48ull * kNoAllocPaths,
-    64ull * kNoAllocPaths,              // hit
-    80ull * kNoAllocPaths,              // queue 0  4 B per path
-    84ull * kNoAllocPaths,              // queue 1
-    88ull * kNoAllocPaths,              // shadow requests 48 B per path
-    136ull * kNoAllocPaths,             // counters (C_COUNT words)
-    136ull * kNoAllocPaths + 128,       // wave descriptor (uint4)
-    136ull * kNoAllocPaths + 160,       // its one segment (WaveSeg)
-    136ull * kNoAllocPaths + 192,       // ray counts (2 x u64)
-    136ull * kNoAllocPaths + 256,       // the view (DevView)
-};
-constexpr size_t kNoAllocBytes = 136ull * kNoAllocPaths + 512;
-static_assert(sizeof(WaveSeg) == 32 && sizeof(DevView) <= 256 && C_COUNT * 4 <= 128, "no-alloc scratch layout");
+constexpr size_t kNoAllocBytes = 16ull * kNoAllocPaths + 16;   // radiance per path, then ray counts (unread)
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 
@@ -1687,17 +1762,6 @@ static int noalloc_scratch(void** out) {
     }
     *out = g_noalloc_addr[dev];
     return CRT_OK;
-}
-
-// Starts a call: clears the counters and ray counts (everything that must
-// start at zero; path state is always written before it is read) and
-// installs the view, the wave's one segment and its descriptor.
-__global__ void wf_noalloc_begin(WaveParams W, uint4 wave, WaveSeg seg, DevView view) {
-    for (int i = 0; i < C_COUNT; ++i) W.counters[i] = 0;
-    W.R.ray_counts[0] = W.R.ray_counts[1] = 0;
-    const_cast<uint4*>(W.waves)[0] = wave;
-    const_cast<WaveSeg*>(W.segs)[0] = seg;
-    const_cast<DevView*>(W.views)[0] = view;
 }
 
 }  // namespace crt
@@ -1731,10 +1795,9 @@ extern "C" int crt_render_tile_noalloc(crt_scene scene, const crt_camera* camera
     void* base = nullptr;
     int st = noalloc_scratch(&base);
     if (st != CRT_OK) return st;
-    unsigned char* b = static_cast<unsigned char*>(base);
-    WaveParams W{};
-    RenderParams& R = W.R;
+    float4* color = static_cast<float4*>(base);
     const bool f32 = uses_f32_nodes(scene, o.node_format);
+    RenderParams R{};
     R.S = scene->view(f32);
     R.cam = to_device_camera(*camera);
     R.accum = reinterpret_cast<float4*>(d_accum);
@@ -1746,41 +1809,8 @@ extern "C" int crt_render_tile_noalloc(crt_scene scene, const crt_camera* camera
     R.nspp = nspp;
     R.max_depth = o.max_depth;
     R.ka_scale = 3.0f * scene->dev.lights_area;
-    R.ray_counts = reinterpret_cast<unsigned long long*>(b + kNoAllocOff[11]);
-    W.views = reinterpret_cast<const DevView*>(b + kNoAllocOff[12]);
-    W.st_od = reinterpret_cast<float4*>(b + kNoAllocOff[0]);   // with [1]: 32 B per path
-    W.st_cm = reinterpret_cast<float4*>(b + kNoAllocOff[2]);   // with [3]: 32 B per path
-    W.hit = reinterpret_cast<float4*>(b + kNoAllocOff[4]);
-    W.queue[0] = reinterpret_cast<uint32_t*>(b + kNoAllocOff[5]);
-    W.queue[1] = reinterpret_cast<uint32_t*>(b + kNoAllocOff[6]);
-    W.shadow = reinterpret_cast<float4*>(b + kNoAllocOff[7]);
-    W.counters = reinterpret_cast<uint32_t*>(b + kNoAllocOff[8]);
-    W.waves = reinterpret_cast<const uint4*>(b + kNoAllocOff[9]);
-    W.segs = reinterpret_cast<const WaveSeg*>(b + kNoAllocOff[10]);
-    W.prof = nullptr;
-    W.stack_depth = (int)traversal_stack(o);
-    W.queue_chunk = queue_chunk(o);
-    W.refill_busy = refill_busy(o);
-    W.octant = false;   // the scratch holds single-region queues
-    W.capacity = kNoAllocPaths;
-    const WaveGrids G = wave_grids(kNoAllocPaths, o.flags, f32, traversal_block(o), W.stack_depth);
-    cudaStream_t s = (cudaStream_t)stream;
-    DevView view;
-    view.cam = R.cam;
-    view.width = width;
-    view.height = height;
-    view.view_id = o.view_id;
-    view.pix_off = 0;
-    const WaveSeg seg{0, pixel0, pixel0 + pixel_count, spp0, spp0 + nspp, 0, 0, 0};
-    wf_noalloc_begin<<<1, 1, 0, s>>>(W, make_uint4(0, 1, pixel_count * nspp, pixel_count), seg, view);
-    wf_generate<false><<<G.gen, kWaveBlock, 0, s>>>(W);
-    for (uint32_t k = 0; k < o.max_depth; ++k) {
-        G.extend<<<G.ext, G.tblock, G.tsmem, s>>>(W);
-        wf_shade<false, false><<<G.gen, kWaveBlock, 0, s>>>(W);
-        G.shadow<<<G.shd, G.tblock, G.tsmem, s>>>(W);
-        wf_flip<<<1, 1, 0, s>>>(W);
-    }
-    wf_accumulate<<<G.acc, 256, 0, s>>>(W);
+    R.ray_counts = reinterpret_cast<unsigned long long*>(color + kNoAllocPaths);
+    launch_paths(R, f32, pixel0, pixel_count, color, (cudaStream_t)stream);
     CRT_CUDA(cudaGetLastError());
     return CRT_OK;
 }
