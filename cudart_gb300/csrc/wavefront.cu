@@ -485,9 +485,7 @@ __global__ void __maxnreg__(CRT_TRAVERSAL_REGS) wf_extend(WaveParams W) {
 // request and its next direction.  ADJ: the adjoint replay, the same bounce
 // with gradient hooks summed into grad_sh.
 template <bool ADJ>
-CRT_D void shade_entry(const WaveParams& W, const QueueView& q, uint32_t i, float* grad_sh, uint32_t& path,
-                       bool& alive, ShadowReq& sr, float3& dir) {
-    path = q.at(i);
+CRT_D void shade_entry(const WaveParams& W, uint32_t path, float* grad_sh, bool& alive, ShadowReq& sr, float3& dir) {
     float4 o, d, c, m;
     ld_pair(W.st_od + 2ull * path, o, d);
     ld_pair(W.st_cm + 2ull * path, c, m);
@@ -559,13 +557,18 @@ CRT_D uint32_t octant_of(float3 d) {
 // octahedral map of the sphere.  A window entry packs (bin, rank in bin)
 // into 16 bits.  Measured (1080p and mixed scenes, FP32 nodes, against no
 // sort): 24 bins +13.6% / +7.8%, 5 x 5 +15.4% / +7.1%, 7 x 7 +16.2% / +7.4%;
-// windows of 2048 entries lost 2-4% to 1024.
+// windows of 2048 entries lost 2-4% to 1024.  Halving the windows of queues
+// shorter than kSortRounds of them per resident block: Cornell box 512x512 x 16
+// 2.39 -> 2.32 ms at 4 (2: 2.38, 8: 2.34), material inversion step 51.0 -> 50.6 (8:
+// 51.3), nothing at 16M-path waves.  Prefetching the next entry's state into L2
+// or L1 lost 3-7%: other sets' kernels already fill the waits.
 #ifndef CRT_SORT_ITERS
 #define CRT_SORT_ITERS 8
 #endif
 #ifndef CRT_SORT_BINNING
 #define CRT_SORT_BINNING 7
 #endif
+constexpr uint32_t kSortRounds = 4;
 constexpr uint32_t kSortIters = CRT_SORT_ITERS, kSortWin = kWaveBlock * kSortIters;
 constexpr uint32_t kSortBinsUsed = CRT_SORT_BINNING == 0 ? 24u : CRT_SORT_BINNING * CRT_SORT_BINNING;
 constexpr uint32_t kSortBins = kSortBinsUsed <= 32u ? 32u : 64u;    // one or two bins per lane in the scan
@@ -607,10 +610,10 @@ __global__ void __maxnreg__(ADJ ? CRT_SHADE_REGS + 32 : CRT_SHADE_REGS) wf_shade
     if (ADJ) zero_grad_block(grad_sh, W.n_mats);
     const uint32_t cur = W.counters[C_CUR];
     const uint32_t n = W.counters[cur];
-    __shared__ uint32_t pre_sh[9];
-    const QueueView q = queue_view(W, cur, pre_sh);
     uint32_t* qn = W.queue[cur ^ 1u];
     if (!SORT) {
+        __shared__ uint32_t pre_sh[9];
+        const QueueView q = queue_view(W, cur, pre_sh);
         const uint32_t end = (n + 31u) & ~31u;   // whole warps stay converged for the ballots
         for (uint32_t i = blockIdx.x * kWaveBlock + threadIdx.x; i < end; i += gridDim.x * kWaveBlock) {
             bool alive = false;
@@ -618,7 +621,10 @@ __global__ void __maxnreg__(ADJ ? CRT_SHADE_REGS + 32 : CRT_SHADE_REGS) wf_shade
             ShadowReq sr;
             sr.valid = false;
             float3 dir = f3(0.f, 0.f, 0.f);
-            if (i < n) shade_entry<ADJ>(W, q, i, grad_sh, path, alive, sr, dir);
+            if (i < n) {
+                path = q.at(i);
+                shade_entry<ADJ>(W, path, grad_sh, alive, sr, dir);
+            }
             if (W.octant) {
                 const uint32_t oct = octant_of(dir);
                 const uint32_t slot = warp_append_keyed(&W.counters[cur ? C_OCT0 : C_OCT1], alive, oct);
@@ -638,17 +644,28 @@ __global__ void __maxnreg__(ADJ ? CRT_SHADE_REGS + 32 : CRT_SHADE_REGS) wf_shade
         constexpr uint32_t kNone = 0xFFFFu, kRankMask = (1u << kRankBits) - 1u;
         __shared__ uint16_t s_ext[kSortWin], s_shd[kSortWin];
         __shared__ uint32_t s_cnt[2 * kSortBins];
-        for (uint32_t w0 = blockIdx.x * kSortWin; w0 < n; w0 += gridDim.x * kSortWin) {
+        // iterations of a window: fewer when the queue holds less than
+        // kSortRounds windows for every resident block (a window of 1024 takes
+        // some 85 us, so the last blocks ran alone and short queues left most of
+        // the chip idle)
+        uint32_t iters = kSortIters;
+        while (iters > 1 && n < gridDim.x * kWaveBlock * iters * kSortRounds) iters >>= 1;
+        const uint32_t win = kWaveBlock * iters;
+        for (uint32_t w0 = blockIdx.x * win; w0 < n; w0 += gridDim.x * win) {
             for (uint32_t k = threadIdx.x; k < 2 * kSortBins; k += kWaveBlock) s_cnt[k] = 0;
             __syncthreads();
-            for (uint32_t it = 0; it < kSortIters; ++it) {
+#pragma unroll 1   // unrolled, 300 bytes spill
+            for (uint32_t it = 0; it < iters; ++it) {
                 const uint32_t j = it * kWaveBlock + threadIdx.x, i = w0 + j;
                 bool alive = false;
                 uint32_t path = 0;
                 ShadowReq sr;
                 sr.valid = false;
                 float3 dir = f3(0.f, 0.f, 0.f);
-                if (i < n) shade_entry<ADJ>(W, q, i, grad_sh, path, alive, sr, dir);
+                if (i < n) {
+                    path = W.queue[cur][i];
+                    shade_entry<ADJ>(W, path, grad_sh, alive, sr, dir);
+                }
                 const uint32_t ek = alive ? direction_bin(dir) : 0u;
                 const uint32_t sk = sr.valid ? (sr.light_face % kSortBinsUsed) : 0u;
                 const uint32_t er = warp_append_keyed(s_cnt, alive, ek, kSortBins);
@@ -697,10 +714,11 @@ __global__ void __maxnreg__(ADJ ? CRT_SHADE_REGS + 32 : CRT_SHADE_REGS) wf_shade
                 }
             }
             __syncthreads();
-            for (uint32_t it = 0; it < kSortIters; ++it) {
+#pragma unroll 1
+            for (uint32_t it = 0; it < iters; ++it) {
                 const uint32_t j = it * kWaveBlock + threadIdx.x, i = w0 + j;
                 const uint32_t e = s_ext[j], sh = s_shd[j];
-                if (e != kNone) qn[s_cnt[e >> kRankBits] + (e & kRankMask)] = q.at(i);
+                if (e != kNone) qn[s_cnt[e >> kRankBits] + (e & kRankMask)] = W.queue[cur][i];
                 if (sh != kNone) W.shadow_q[s_cnt[kSortBins + (sh >> kRankBits)] + (sh & kRankMask)] = i;
             }
             __syncthreads();   // the next window reuses the shared arrays
@@ -1090,6 +1108,7 @@ static WaveParams wave_params(crt_render r, WaveSet& set) {
 
 struct WaveGrids {
     int gen, ext, shd, acc, cnt;
+    int sha, sha_adj;    // shade and its adjoint: resident blocks
     int tblock;          // extend / shadow threads per block
     size_t tsmem;        // their dynamic shared memory (traversal stacks)
     WaveKernel extend, shadow, extend_count, shadow_count;
@@ -1112,6 +1131,8 @@ static WaveGrids wave_grids(uint32_t capacity, uint32_t flags, bool f32, uint32_
     cudaFuncSetAttribute((const void*)g.extend, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.tsmem);
     cudaFuncSetAttribute((const void*)g.shadow, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.tsmem);
     g.gen = grid_for(capacity, kWaveBlock, 16);
+    g.sha = std::min(g.gen, persistent_grid((const void*)g.shade, kWaveBlock, 0));
+    g.sha_adj = std::min(g.gen, persistent_grid((const void*)g.shade_adj, kWaveBlock, 0));
     g.ext = persistent_grid((const void*)g.extend, g.tblock, g.tsmem);
     g.shd = persistent_grid((const void*)g.shadow, g.tblock, g.tsmem);
     g.cnt = persistent_grid((const void*)g.extend_count, kWaveBlock, 0);
@@ -1140,7 +1161,7 @@ static void enqueue_wave_body(const WaveParams& W, const WaveGrids& G, uint32_t 
     for (uint32_t b = 0; b < max_depth; ++b) {
         G.extend<<<G.ext, G.tblock, G.tsmem, s>>>(W);
         if (!s2) {
-            G.shade<<<G.gen, kWaveBlock, 0, s>>>(W);
+            G.shade<<<G.sha, kWaveBlock, 0, s>>>(W);
             G.shadow<<<G.shd, G.tblock, G.tsmem, s>>>(W);
             wf_flip<<<1, 1, 0, s>>>(W);
             continue;
@@ -1149,7 +1170,7 @@ static void enqueue_wave_body(const WaveParams& W, const WaveGrids& G, uint32_t 
             cudaStreamWaitEvent(s, shadowed, 0);   // shadow(b - 1) is done
             wf_flip_shadow<<<1, 1, 0, s>>>(W);
         }
-        G.shade<<<G.gen, kWaveBlock, 0, s>>>(W);
+        G.shade<<<G.sha, kWaveBlock, 0, s>>>(W);
         cudaEventRecord(shaded, s);
         cudaStreamWaitEvent(s2, shaded, 0);
         G.shadow<<<G.shd, G.tblock, G.tsmem, s2>>>(W);
@@ -1572,7 +1593,7 @@ static int capture_adjoint_graph(crt_render r, WaveSet& set, const float4* adj, 
         wf_generate<true><<<G.gen, kWaveBlock, 0, cap>>>(W);  // replay
         for (uint32_t b = 0; b < r->opts.max_depth; ++b) {
             G.extend<<<G.ext, G.tblock, G.tsmem, cap>>>(W);
-            G.shade_adj<<<G.gen, kWaveBlock, A.shade_smem, cap>>>(W);
+            G.shade_adj<<<G.sha_adj, kWaveBlock, A.shade_smem, cap>>>(W);
             A.shadow<<<A.shd, G.tblock, A.shadow_smem, cap>>>(W);
             wf_flip<<<1, 1, 0, cap>>>(W);
         }
@@ -1690,7 +1711,7 @@ int wavefront_profile_pass(crt_render r, const std::vector<ViewWork>& work, crt_
                 out->extend_rays_by_bounce[bb] += counter(counter(C_CUR));
                 wf_reset_count_fetch<<<1, 1, 0, s>>>(W);
                 G.extend_count<<<G.cnt, kWaveBlock, 0, s>>>(W);
-                timed(2, [&] { G.shade<<<G.gen, kWaveBlock, 0, s>>>(W); });
+                timed(2, [&] { G.shade<<<G.sha, kWaveBlock, 0, s>>>(W); });
                 out->shadow_ms_by_bounce[bb] += timed(3, [&] { G.shadow<<<G.shd, G.tblock, G.tsmem, s>>>(W); });
                 out->shadow_rays_by_bounce[bb] += counter(C_SHADOW);
                 wf_reset_count_fetch<<<1, 1, 0, s>>>(W);
