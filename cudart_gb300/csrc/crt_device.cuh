@@ -479,46 +479,6 @@ CRT_D bool traverse(const DevScene& S, float3 o, float3 d, float tmin, Hit& h, i
     return T.occluded;
 }
 
-// Warp-local pool of queue entries for persistent kernels: lanes whose ray
-// finished take the next entries at once, and the warp claims 32 more from
-// the global counter only when the pool runs dry.
-struct WarpPool {
-    uint32_t next, end;      // warp-uniform
-    bool exhausted;
-
-    CRT_D void init() { next = end = 0; exhausted = false; }
-
-    // Returns the queue index for this lane (or UINT32_MAX) when `want`.
-    CRT_D uint32_t take(bool want, uint32_t* counter, uint32_t n) {
-        const uint32_t lane = threadIdx.x & 31u;
-        const uint32_t need = __ballot_sync(0xFFFFFFFFu, want);
-        if (!need || exhausted) return UINT32_MAX;
-        const uint32_t k = __popc(need);
-        const uint32_t rank = __popc(need & ((1u << lane) - 1u));
-        const uint32_t have = end - next;
-        uint32_t mine = UINT32_MAX;
-        if (want && rank < have) mine = next + rank;
-        if (k <= have) {
-            next += k;
-        } else {
-            uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(counter, 32u);
-            base = __shfl_sync(0xFFFFFFFFu, base, 0);
-            if (base >= n) {
-                exhausted = true;
-                next = end;
-            } else {
-                const uint32_t chunk_end = base + 32u < n ? base + 32u : n;
-                if (want && rank >= have && base + (rank - have) < chunk_end) mine = base + (rank - have);
-                const uint32_t used = k - have;
-                next = base + used < chunk_end ? base + used : chunk_end;
-                end = chunk_end;
-            }
-        }
-        return mine;
-    }
-};
-
 // ---------------------------------------------------------------------------
 // Estimator pieces (src/renderer/renderer.cu:119-262 and helpers)
 // ---------------------------------------------------------------------------

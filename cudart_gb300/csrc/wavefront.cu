@@ -397,51 +397,84 @@ __global__ void __launch_bounds__(kWaveBlock) wf_generate(WaveParams W) {
     }
 }
 
-// Persistent work loop shared by the extend and shadow kernels.  REFILL: a
-// lane whose ray finished takes the next queue entry at once (warp-local
-// pool, one global atomic per 32 entries).  Otherwise a warp takes 32 entries
-// and runs all of them to completion before taking more.  Job supplies
-// start(i) (initialise the lane's traversal for queue entry i), step() and
-// finish().
-template <bool REFILL, class Job>
-CRT_D void persistent_loop(uint32_t n, uint32_t* fetch, uint32_t chunk, uint32_t refill_busy, Job& job) {
-    if (REFILL) {
-        // idle lanes take new entries together, once at most `refill_busy`
-        // lanes of the warp are still busy (31: as soon as one is idle)
-        bool active = false;
-        WarpPool pool;
-        pool.init();
-        for (;;) {
-            if ((uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, active)) <= refill_busy) {
-                const uint32_t i = pool.take(!active, fetch, n);
-                if (i != UINT32_MAX) {
-                    job.start(i);
-                    active = true;
-                }
-                if (!__any_sync(0xFFFFFFFFu, active)) break;
-            }
-            if (active && job.step()) {
-                job.finish();
-                active = false;
-            }
+// Work loops of the extend and shadow kernels.  Job supplies start(i)
+// (initialise the lane's traversal for queue entry i), step(), finish() and
+// visits() (node visits of the finished ray).
+//
+// refill_loop: the warp runs until at most `refill_busy` lanes are still busy;
+// then the idle lanes store their results and take the next entries together,
+// neighbours in the queue (taking them from a warp-local pool of 32 instead mixed
+// entries claimed at different times into one warp and cost 10%).
+template <class Job>
+CRT_D void refill_loop(uint32_t n, uint32_t* fetch, uint32_t refill_busy, Job& job) {
+    const uint32_t lane = threadIdx.x & 31u;
+    bool busy = false, done = false;
+    for (;;) {
+        const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !busy);
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(fetch, __popc(idle));
+        base = __shfl_sync(0xFFFFFFFFu, base, 0);
+        if (base >= n || n - base <= (uint32_t)__popc(idle)) refill_busy = 0;   // the queue is empty: run what is left
+        if (!busy) {
+            if (done) job.finish();
+            const uint32_t k = __popc(idle & ((1u << lane) - 1u));
+            busy = done = base < n && k < n - base;
+            if (busy) job.start(base + k);
         }
-    } else {
-        // each warp claims `chunk` entries (a multiple of 32) per atomic
-        const uint32_t lane = threadIdx.x & 31u;
-        for (;;) {
-            uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(fetch, chunk);
-            base = __shfl_sync(0xFFFFFFFFu, base, 0);
-            if (base >= n) break;
-            const uint32_t end = min(base + chunk, n);
-            for (uint32_t i = base + lane; i < end; i += 32u) {
+        if (!__any_sync(0xFFFFFFFFu, busy)) break;
+        do {
+            if (busy) busy = !job.step();
+        } while ((uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, busy)) > refill_busy);
+    }
+}
+
+// batch_loop: each warp claims `chunk` entries (a multiple of 32) per atomic and
+// runs 32 at a time to completion.  That keeps rays that start alike together,
+// but the warp waits for its longest ray.  ADAPT: after kAdaptBatches batches the
+// warp compares its lanes' visits with 32 times its longest rays': below one
+// half it goes on with refill_loop.  Measured (a pass's extension / shadow
+// traversals, batch -> refill at 16 busy lanes): mixed scene, half at 0.33 to 0.54,
+// 15.6 -> 13.9 / 6.5 -> 5.3 ms; 2.17M triangles, 0.56 and above, 7.1 -> 8.2 / 2.35 ->
+// 2.8 ms; Cornell box, 0.50 but under two visits per ray, 0.82 -> 0.90 ms (hence at
+// least kAdaptVisits per ray).  1001x563 x 32, mixed scene: 36.9 ms without,
+// deciding after 8 / 4 / 2 batches 32.9 / 32.4 / 32.1, refilling at 12 / 16 / 20 busy
+// lanes 33.1 / 32.4 / 32.0.
+constexpr uint32_t kAdaptBatches = 2, kAdaptVisits = 3, kAdaptBusy = 20;
+template <bool ADAPT, class Job>
+CRT_D void batch_loop(uint32_t n, uint32_t* fetch, uint32_t chunk, Job& job) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t batches = 0, sum = 0, longest = 0;
+    for (;;) {
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(fetch, chunk);
+        base = __shfl_sync(0xFFFFFFFFu, base, 0);
+        if (base >= n) return;
+        const uint32_t end = min(base + chunk, n);
+        for (uint32_t first = base; first < end; first += 32u) {
+            const uint32_t i = first + lane;
+            uint32_t v = 0;
+            if (i < end) {
                 job.start(i);
                 while (!job.step()) {
                 }
                 job.finish();
+                v = job.visits();
+            }
+            if (ADAPT) {
+                ++batches;
+                sum += __reduce_add_sync(0xFFFFFFFFu, v);
+                longest += __reduce_max_sync(0xFFFFFFFFu, v);
             }
         }
+        if (ADAPT && batches >= kAdaptBatches && sum < 16u * longest && sum >= 32u * kAdaptVisits * batches) break;
     }
+    refill_loop(n, fetch, kAdaptBusy, job);
+}
+
+template <bool REFILL, bool WHOLE_LEAF, class Job>
+CRT_D void persistent_loop(uint32_t n, uint32_t* fetch, uint32_t chunk, uint32_t refill_busy, Job& job) {
+    if (REFILL) refill_loop(n, fetch, refill_busy, job);
+    else batch_loop<WHOLE_LEAF>(n, fetch, chunk, job);
 }
 
 template <bool WHOLE_LEAF, bool F32>
@@ -460,6 +493,7 @@ struct ExtendJob {
         T.init(xyz(o), xyz(d), kEps, FLT_MAX, -1, st, W.R.S.max_visits);
     }
     CRT_D bool step() { return T.step(W.R.S, st, nullptr); }
+    CRT_D uint32_t visits() const { return T.visits - (kVisitCeiling - W.R.S.max_visits); }
     CRT_D void finish() {
         W.hit[path] = make_float4(T.h.t, __int_as_float(T.h.face), T.h.u, T.h.v);
         ++rays;
@@ -476,7 +510,7 @@ __global__ void __maxnreg__(CRT_TRAVERSAL_REGS) wf_extend(WaveParams W) {
     const uint32_t cur = W.counters[C_CUR];
     __shared__ uint32_t pre_sh[9];
     ExtendJob<WHOLE_LEAF, F32> job(W, queue_view(W, cur, pre_sh), st);
-    persistent_loop<REFILL>(W.counters[cur], &W.counters[C_FETCH_EXT], W.queue_chunk, W.refill_busy, job);
+    persistent_loop<REFILL, WHOLE_LEAF>(W.counters[cur], &W.counters[C_FETCH_EXT], W.queue_chunk, W.refill_busy, job);
     count_rays(W.R.ray_counts, job.rays, 0);
 }
 
@@ -743,6 +777,7 @@ struct ShadowJob {
         T.init(xyz(e[0]), xyz(b), kEps, b.w, (int32_t)__float_as_uint(e[2].w), st, W.R.S.max_visits);
     }
     CRT_D bool step() { return T.step(W.R.S, st, nullptr); }
+    CRT_D uint32_t visits() const { return T.visits - (kVisitCeiling - W.R.S.max_visits); }
     // a visible light adds the request's contribution to the path colour
     CRT_D void finish() {
         ++rays;
@@ -772,7 +807,7 @@ __global__ void __maxnreg__(CRT_TRAVERSAL_REGS) wf_shadow_adj(WaveParams W) {
     StackSpill overflow;
     Stack st(crt_stacks, overflow, blockDim.x, W.stack_depth);
     ShadowJob<true, F32, true> job(W, st, grad);
-    persistent_loop<false>(W.counters[C_SHADOW], &W.counters[C_FETCH_SHD], W.queue_chunk, 31u, job);
+    persistent_loop<false, true>(W.counters[C_SHADOW], &W.counters[C_FETCH_SHD], W.queue_chunk, 31u, job);
     count_rays(W.R.ray_counts, 0, job.rays);
     flush_grad_block(W, grad);
 }
@@ -782,7 +817,7 @@ __global__ void __maxnreg__(CRT_TRAVERSAL_REGS) wf_shadow(WaveParams W) {
     StackSpill overflow;
     Stack st(crt_stacks, overflow, blockDim.x, W.stack_depth);
     ShadowJob<WHOLE_LEAF, F32> job(W, st);
-    persistent_loop<REFILL>(W.counters[C_SHADOW], &W.counters[C_FETCH_SHD], W.queue_chunk, W.refill_busy, job);
+    persistent_loop<REFILL, WHOLE_LEAF>(W.counters[C_SHADOW], &W.counters[C_FETCH_SHD], W.queue_chunk, W.refill_busy, job);
     count_rays(W.R.ray_counts, 0, job.rays);
 }
 
