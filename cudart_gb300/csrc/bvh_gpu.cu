@@ -64,11 +64,10 @@ struct GDec {
     uint8_t pad;
 };
 
-// Children of one wide node, in the order the collapse picked them.
+// One wide node: the binary node in each slot (-1: empty) and its bases.
 struct GWide {
-    int32_t nch;
-    int32_t ch[8];
-    int32_t slot_of[8];
+    int32_t child[8];
+    uint32_t child_base, tri_base;
 };
 
 __device__ __forceinline__ uint32_t float_order(float f) {
@@ -104,12 +103,15 @@ __global__ void k_max_abs(const float* __restrict__ v1, const float* __restrict_
 
 // Conservative triangle boxes and centroids exactly as the host build forms
 // them (FP64 bounds minus / plus the margin, rounded outward to FP32), and
-// the centroid bounds.
+// the centroid bounds, reduced per block before the atomics (one set of six per
+// triangle took 300 us of 2.17M triangles' 383 us here).
 __global__ void k_tri_boxes(const float* __restrict__ v1, const float* __restrict__ e1, const float* __restrict__ e2,
                             uint32_t n, float margin, GBox* __restrict__ tbox, float* __restrict__ cent,
                             uint32_t* __restrict__ cbounds) {
+    uint32_t lo6[3] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, hi6[3] = {0u, 0u, 0u};
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
         GBox b;
+#pragma unroll
         for (int k = 0; k < 3; ++k) {
             const double a = v1[3ull * t + k];
             const double bb = a + (double)e1[3ull * t + k];
@@ -122,11 +124,25 @@ __global__ void k_tri_boxes(const float* __restrict__ v1, const float* __restric
             b.hi[k] = fhi;
             const float cc = 0.5f * (flo + fhi);
             cent[3ull * t + k] = cc;
-            atomicMin(&cbounds[k], float_order(cc));
-            atomicMax(&cbounds[3 + k], float_order(cc));
+            lo6[k] = min(lo6[k], float_order(cc));
+            hi6[k] = max(hi6[k], float_order(cc));
         }
         tbox[t] = b;
     }
+    __shared__ uint32_t sh[6];
+    if (threadIdx.x < 6) sh[threadIdx.x] = threadIdx.x < 3 ? 0xFFFFFFFFu : 0u;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const uint32_t l = __reduce_min_sync(0xFFFFFFFFu, lo6[k]), h = __reduce_max_sync(0xFFFFFFFFu, hi6[k]);
+        if ((threadIdx.x & 31u) == 0) {
+            atomicMin(&sh[k], l);
+            atomicMax(&sh[3 + k], h);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 3) atomicMin(&cbounds[threadIdx.x], sh[threadIdx.x]);
+    else if (threadIdx.x < 6) atomicMax(&cbounds[threadIdx.x], sh[threadIdx.x]);
 }
 
 // Spreads the low 21 bits of x to every third bit of a 63-bit code.
@@ -171,90 +187,164 @@ __global__ void k_leaves(const GBox* __restrict__ tbox, const uint32_t* __restri
     if (i >= n) return;
     GNode& lf = nodes[n - 1 + i];
     lf.box = tbox[perm[i]];
-    lf.left = lf.right = -1;
+    lf.left = lf.right = lf.parent = -1;
     lf.first = (uint32_t)i;
     lf.count = 1;
 }
 
-// PLOC nearest neighbour: for cluster i of m (in Morton order), the cluster
-// j within kRadius places whose merged box has the least half area.  Pairs
-// are ordered by (area, |i - j|, min(i, j) odd, min(i, j)): a total order on
-// unordered pairs, so the best pair overall is always mutual and every
-// iteration merges; among equal boxes (2k, 2k + 1) pair up, so even a scene
-// of identical triangles halves its clusters every iteration.
-__global__ void k_ploc_nn(const int32_t* __restrict__ clusters, int m, const GNode* __restrict__ nodes,
-                          int32_t* __restrict__ nn, int n, uint32_t* err) {
-    __shared__ GBox tile[kBlock + 2 * kRadius];
-    const int b0 = blockIdx.x * kBlock;
-    const int lo = max(0, b0 - kRadius), hi = min(m, b0 + kBlock + kRadius);   // [lo, hi) staged
-    for (int k = lo + (int)threadIdx.x; k < hi; k += kBlock) {
-        const int32_t c = clusters[k];
+// Clusters left and the next node id of one PLOC iteration.
+struct PlocState {
+    int32_t m, next_id;
+};
+
+// PLOC pairs: for cluster i of m (in Morton order), the cluster j within
+// kRadius places whose merged box has the least half area; i and j pair if each
+// is the other's.  Pairs are ordered by (area, |i - j|, min(i, j) odd, min(i,
+// j)): a total order on unordered pairs, so the best pair overall is always
+// mutual and every iteration merges; among equal boxes (2k, 2k + 1) pair up, so
+// even a scene of identical triangles halves its clusters every iteration.
+// A block also finds the neighbours of the kRadius clusters on either side of
+// its own, so it knows which of its clusters pair, writes pair[i] (j or -1) and
+// counts its survivors (high word) and new nodes (low word).
+__global__ void __launch_bounds__(kBlock) k_ploc_pairs(const int32_t* __restrict__ clusters,
+                                                       const PlocState* __restrict__ state,
+                                                       const GNode* __restrict__ nodes, int32_t* __restrict__ pair,
+                                                       uint64_t* __restrict__ counts, int n, uint32_t* err) {
+    constexpr int kTile = kBlock + 4 * kRadius, kNear = kBlock + 2 * kRadius;
+    __shared__ GBox tile[kTile];
+    __shared__ int near[kNear];
+    const int m = state->m;
+    const int b0 = (int)(blockIdx.x * kBlock);
+    if (b0 >= m) return;   // the whole block
+    const int t0 = b0 - 2 * kRadius;   // cluster of tile[0]
+    for (int k = (int)threadIdx.x; k < kTile; k += kBlock) {
+        const int i = t0 + k;
+        if (i < 0 || i >= m) continue;
+        const int32_t c = clusters[i];
         if (c < 0 || c > 2 * n - 2) {   // never expected; keeps the read in bounds
             atomicOr(err, 1u);
-            tile[k - lo] = GBox{{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
+            tile[k] = GBox{{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
         } else {
-            tile[k - lo] = nodes[c].box;
+            tile[k] = nodes[c].box;
         }
     }
     __syncthreads();
-    const int i = b0 + (int)threadIdx.x;
-    if (i >= m) return;
-    const GBox bi = tile[i - lo];
-    float best = FLT_MAX;
-    int bj = -1, bdist = INT_MAX, bodd = 1, bmin = INT_MAX;
-    const int j0 = max(0, i - kRadius), j1 = min(m - 1, i + kRadius);
-    for (int j = j0; j <= j1; ++j) {
-        if (j == i) continue;
-        GBox u = bi;
-        grow(u, tile[j - lo]);
-        const float d = half_area(u);
-        const int dist = abs(i - j), mn = min(i, j), odd = mn & 1;
-        const bool better =
-            d < best || (d == best && (dist < bdist || (dist == bdist && (odd < bodd || (odd == bodd && mn < bmin)))));
-        if (better) {
-            best = d;
-            bj = j;
-            bdist = dist;
-            bodd = odd;
-            bmin = mn;
+    const int n0 = b0 - kRadius;       // cluster of near[0]
+    for (int k = (int)threadIdx.x; k < kNear; k += kBlock) {
+        const int i = n0 + k;
+        int bj = -1;
+        if (i >= 0 && i < m) {
+            const GBox bi = tile[i - t0];
+            float best = FLT_MAX;
+            int bdist = INT_MAX, bodd = 1, bmin = INT_MAX;
+            const int j0 = max(0, i - kRadius), j1 = min(m - 1, i + kRadius);
+            for (int j = j0; j <= j1; ++j) {
+                if (j == i) continue;
+                GBox u = bi;
+                grow(u, tile[j - t0]);
+                const float d = half_area(u);
+                const int dist = abs(i - j), mn = min(i, j), odd = mn & 1;
+                const bool better = d < best || (d == best && (dist < bdist || (dist == bdist && (odd < bodd || (odd == bodd && mn < bmin)))));
+                if (better) {
+                    best = d;
+                    bj = j;
+                    bdist = dist;
+                    bodd = odd;
+                    bmin = mn;
+                }
+            }
         }
+        near[k] = bj;
     }
-    nn[i] = bj;
+    __syncthreads();
+    const int i = b0 + (int)threadIdx.x;
+    bool survive = false, create = false;
+    if (i < m) {
+        const int j = near[i - n0];
+        const bool mutual = j >= 0 && near[j - n0] == i;
+        pair[i] = mutual ? j : -1;
+        create = mutual && i < j;
+        survive = !mutual || i < j;
+    }
+    const int ns = __syncthreads_count(survive), nc = __syncthreads_count(create);
+    if (threadIdx.x == 0) counts[blockIdx.x] = ((uint64_t)ns << 32) | (uint64_t)nc;
 }
 
-// Merge flags, packed for one 64-bit scan: high word = cluster survives
-// (kept or merged into), low word = a new node is created here.
-__global__ void k_ploc_flags(const int32_t* __restrict__ nn, int m, uint64_t* __restrict__ flags) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m) return;
-    const int j = nn[i];
-    const bool mutual = j >= 0 && j < m && nn[j] == i;
-    const bool create = mutual && i < j;
-    const bool survive = !mutual || i < j;
-    flags[i] = ((uint64_t)survive << 32) | (uint64_t)create;
+// Exclusive sums of the block counts in place (one block), and the next
+// iteration's state.
+__global__ void __launch_bounds__(1024) k_ploc_scan(uint64_t* __restrict__ counts, const PlocState* __restrict__ state,
+                                                    PlocState* __restrict__ next, uint32_t* err) {
+    __shared__ uint64_t warp_sum[32];
+    const int m = state->m, blocks = (m + kBlock - 1) / kBlock;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint64_t carry = 0;
+    for (int b0 = 0; b0 < blocks; b0 += 1024) {
+        const int b = b0 + (int)threadIdx.x;
+        const uint64_t v = b < blocks ? counts[b] : 0;
+        uint64_t x = v;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint64_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+            if ((int)lane >= o) x += y;
+        }
+        if (lane == 31) warp_sum[warp] = x;
+        __syncthreads();
+        if (warp == 0) {
+            uint64_t w = warp_sum[lane];
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint64_t y = __shfl_up_sync(0xFFFFFFFFu, w, o);
+                if ((int)lane >= o) w += y;
+            }
+            warp_sum[lane] = w;
+        }
+        __syncthreads();
+        const uint64_t before = carry + (warp ? warp_sum[warp - 1] : 0) + x - v;
+        if (b < blocks) counts[b] = before;
+        carry += warp_sum[31];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        const int32_t survivors = (int32_t)(carry >> 32), merges = (int32_t)(uint32_t)carry;
+        if (survivors + merges != m || (m > 1 && merges == 0) || state->next_id + 1 < merges) atomicOr(err, 1u);
+        next->m = survivors;
+        next->next_id = state->next_id - merges;
+    }
 }
 
-__global__ void k_ploc_init(int32_t* __restrict__ clusters, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) clusters[i] = n - 1 + i;   // every triangle is a cluster
-}
-
-// Creates the merged nodes (ids counting down from `next_id`) and writes the
+// Creates the merged nodes (ids counting down from next_id) and writes the
 // compacted cluster list.
-__global__ void k_ploc_merge(const int32_t* __restrict__ clusters, const int32_t* __restrict__ nn, int m,
-                             const uint64_t* __restrict__ scan, int32_t next_id, GNode* __restrict__ nodes,
-                             int32_t* __restrict__ out, int n, uint32_t* err) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m) return;
-    const int j = nn[i];
-    const bool mutual = j >= 0 && j < m && nn[j] == i;
-    if (mutual && i > j) return;   // merged into cluster j
-    const uint64_t sc = scan[i];
-    const uint32_t pos = (uint32_t)(sc >> 32);
+__global__ void __launch_bounds__(kBlock) k_ploc_merge(const int32_t* __restrict__ clusters,
+                                                       const int32_t* __restrict__ pair,
+                                                       const PlocState* __restrict__ state,
+                                                       const uint64_t* __restrict__ counts, GNode* __restrict__ nodes,
+                                                       int32_t* __restrict__ out, int n, uint32_t* err) {
+    __shared__ uint32_t warp_s[kBlock / 32], warp_c[kBlock / 32];
+    const int m = state->m;
+    const int b0 = (int)(blockIdx.x * kBlock);
+    if (b0 >= m) return;   // the whole block
+    const int i = b0 + (int)threadIdx.x;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const int j = i < m ? pair[i] : -1;
+    const bool create = i < m && j > i, survive = i < m && (j < 0 || j > i);
+    const uint32_t bs = __ballot_sync(0xFFFFFFFFu, survive), bc = __ballot_sync(0xFFFFFFFFu, create);
+    if (lane == 0) {
+        warp_s[warp] = __popc(bs);
+        warp_c[warp] = __popc(bc);
+    }
+    __syncthreads();
+    if (!survive) return;
+    const uint64_t before = counts[blockIdx.x];
+    uint32_t pos = (uint32_t)(before >> 32), made = (uint32_t)before;
+    for (uint32_t w = 0; w < warp; ++w) {
+        pos += warp_s[w];
+        made += warp_c[w];
+    }
+    const uint32_t below = (1u << lane) - 1u;
+    pos += __popc(bs & below);
+    made += __popc(bc & below);
     int32_t id = clusters[i];
-    if (mutual) {
-        id = next_id - (int32_t)(uint32_t)(sc & 0xFFFFFFFFull);
-        const int32_t l = clusters[i], r = clusters[j];
+    if (create) {
+        id = state->next_id - (int32_t)made;
+        const int32_t l = clusters[i], r = j < m ? clusters[j] : -1;
         if (id < 0 || id > n - 2 || l < 0 || r < 0 || l > 2 * n - 2 || r > 2 * n - 2) {
             atomicOr(err, 1u);   // never expected; keeps every write in bounds
             return;
@@ -278,58 +368,73 @@ __global__ void k_ploc_merge(const int32_t* __restrict__ clusters, const int32_t
     out[pos] = id;
 }
 
-// C(x, 1..W) of the collapse, from the children's costs (cost[8 * node + i - 1]).
-__device__ void dp_node(int32_t x, const GNode& nd, const float* L, const float* R, int W, float* C, GDec& d) {
+__global__ void k_ploc_init(int32_t* __restrict__ clusters, int n, PlocState* __restrict__ state) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) clusters[i] = n - 1 + i;   // every triangle is a cluster
+    if (i == 0) *state = PlocState{n, n - 2};
+}
+
+// C(x, 1..W) of the collapse, from the children's costs.
+template <int W>
+__device__ __forceinline__ void dp_node(const GNode& nd, const float* L, const float* R, float* C, GDec& d) {
     const float A = half_area(nd.box);
     const float leafc = nd.count <= kSlotTrisMax ? kTriCost * A * (float)nd.count : FLT_MAX;
-    float D[9];
-    uint8_t K[9];
+    float D[W + 1];
+    int K[W + 1];
+#pragma unroll
     for (int i = 2; i <= W; ++i) {
         D[i] = FLT_MAX;
         K[i] = 1;
+#pragma unroll
         for (int k = 1; k < i; ++k) {
             const float c = L[k - 1] + R[i - k - 1];
             if (c < D[i]) {
                 D[i] = c;
-                K[i] = (uint8_t)k;
+                K[i] = k;
             }
         }
     }
     const float wide = A + D[W];
     d.leaf = leafc <= wide;
-    d.wk = K[W];
+    d.wk = (uint8_t)K[W];
     C[0] = d.leaf ? leafc : wide;
-    d.split[1] = 0;
+    d.split[0] = d.split[1] = 0;
+#pragma unroll
     for (int i = 2; i <= W; ++i) {
         if (D[i] < C[i - 2]) {
             C[i - 1] = D[i];
-            d.split[i] = K[i];
+            d.split[i] = (uint8_t)K[i];
         } else {
             C[i - 1] = C[i - 2];
             d.split[i] = 0;
         }
     }
+#pragma unroll
+    for (int i = W + 1; i < 9; ++i) d.split[i] = 0;
+    d.pad = 0;
 }
 
-__global__ void k_dp_leaves(int n, const GNode* __restrict__ nodes, int W, float* __restrict__ cost,
-                            GDec* __restrict__ dec) {
+// Bottom-up from the leaves: the second child to finish computes its parent.
+// cost[8 * node + i - 1] is C(node, i).  (Loops over W known at compile time
+// keep the tables in registers: with the leaves 0.91 -> 0.36 ms of 2.17M
+// triangles.)
+template <int W>
+__global__ void k_dp_up(int n, const GNode* __restrict__ nodes, float* cost, GDec* __restrict__ dec, uint32_t* flags,
+                        uint32_t* err) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const int x = n - 1 + i;
-    const float c = kTriCost * half_area(nodes[x].box) * (float)nodes[x].count;
-    for (int k = 0; k < W; ++k) cost[8ull * x + k] = c;
-    GDec d;
-    memset(&d, 0, sizeof(d));
-    d.leaf = 1;
-    dec[x] = d;
-}
-
-// Bottom-up: the second child to finish computes its parent.
-__global__ void k_dp_up(int n, const GNode* __restrict__ nodes, int W, float* cost, GDec* __restrict__ dec,
-                        uint32_t* flags, uint32_t* err) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int p = nodes[n - 1 + i].parent;
+    const int leaf = n - 1 + i;
+    {
+        const float c = kTriCost * half_area(nodes[leaf].box) * (float)nodes[leaf].count;
+        float4* to = reinterpret_cast<float4*>(cost + 8ull * leaf);
+        __stcg(to, make_float4(c, c, c, c));
+        if (W > 4) __stcg(to + 1, make_float4(c, c, c, c));
+        GDec d;
+        memset(&d, 0, sizeof(d));
+        d.leaf = 1;
+        dec[leaf] = d;
+    }
+    int p = nodes[leaf].parent;
     for (int climbed = 0; p >= 0; ++climbed) {
         if (p > n - 2 || climbed >= n) {   // never expected; ends the climb
             atomicOr(err, 8u);
@@ -344,14 +449,19 @@ __global__ void k_dp_up(int n, const GNode* __restrict__ nodes, int W, float* co
             return;
         }
         float L[8], R[8], C[8];
-        for (int k = 0; k < W; ++k) {
-            L[k] = __ldcg(&cost[8ull * nd.left + k]);
-            R[k] = __ldcg(&cost[8ull * nd.right + k]);
+        const float4* pl = reinterpret_cast<const float4*>(cost + 8ull * nd.left);
+        const float4* pr = reinterpret_cast<const float4*>(cost + 8ull * nd.right);
+#pragma unroll
+        for (int h = 0; h < W / 4; ++h) {
+            const float4 a = __ldcg(pl + h), b = __ldcg(pr + h);
+            L[4 * h] = a.x; L[4 * h + 1] = a.y; L[4 * h + 2] = a.z; L[4 * h + 3] = a.w;
+            R[4 * h] = b.x; R[4 * h + 1] = b.y; R[4 * h + 2] = b.z; R[4 * h + 3] = b.w;
         }
         GDec d;
-        memset(&d, 0, sizeof(d));
-        dp_node(p, nd, L, R, W, C, d);
-        for (int k = 0; k < W; ++k) __stcg(&cost[8ull * p + k], C[k]);
+        dp_node<W>(nd, L, R, C, d);
+        float4* to = reinterpret_cast<float4*>(cost + 8ull * p);
+#pragma unroll
+        for (int h = 0; h < W / 4; ++h) __stcg(to + h, make_float4(C[4 * h], C[4 * h + 1], C[4 * h + 2], C[4 * h + 3]));
         dec[p] = d;
         p = nd.parent;
     }
@@ -359,183 +469,216 @@ __global__ void k_dp_up(int n, const GNode* __restrict__ nodes, int W, float* co
 
 __device__ __forceinline__ bool wide_slot(const GDec* dec, int32_t x) { return dec[x].leaf == 0; }
 
-// One wide node per thread: the collapse's children, slots by octant.
-__global__ void k_choose(const int32_t* __restrict__ front, uint32_t F, const GNode* __restrict__ nodes,
-                         const GDec* __restrict__ dec, int max_children, GWide* __restrict__ recs,
-                         uint32_t* __restrict__ cnt_int, uint32_t* __restrict__ cnt_tri, int n, uint32_t* err) {
-    const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= F) return;
+// One wide node per 8 lanes: the collapse's children, slots by octant.  The
+// first lane expands the decisions; then lane c holds child c.  (One thread per
+// node kept children and slots in local memory: 0.55 -> 0.32 ms over the levels of
+// 2.17M triangles, and 0.86 -> 0.23 ms for k_emit, which now also runs once.)
+__global__ void __launch_bounds__(kBlock) k_choose(const int32_t* __restrict__ front, uint32_t F,
+                                                   const GNode* __restrict__ nodes, const GDec* __restrict__ dec,
+                                                   int max_children, GWide* __restrict__ recs,
+                                                   uint64_t* __restrict__ counts, int n, uint32_t* err) {
+    __shared__ int32_t kids[kBlock];
+    const uint32_t f = (uint32_t)(((uint64_t)blockIdx.x * kBlock + threadIdx.x) >> 3);
+    const uint32_t lane = threadIdx.x & 7u, group = threadIdx.x & ~7u;
+    const uint32_t mask = 0xFFu << (threadIdx.x & 24u);
+    if (f >= F) return;   // whole groups of 8
     const int32_t x = front[f];
-    GWide w;
     int nch = 0;
-    if (!wide_slot(dec, x)) {
-        w.ch[nch++] = x;                      // a root of at most 3 triangles
-    } else {
-        // expand (node, slots) pairs left to right, as DpCollapse::expand
-        int32_t sn[16];
-        int sb[16];
-        int sp = 0;
-        sn[sp] = nodes[x].right;
-        sb[sp++] = max_children - dec[x].wk;
-        sn[sp] = nodes[x].left;
-        sb[sp++] = dec[x].wk;
-        while (sp > 0) {
-            const int32_t y = sn[--sp];
-            int i = sb[sp];
-            if (y < 0 || y > 2 * n - 2 || i < 1 || i > max_children) { atomicOr(err, 16u); break; }
-            while (i > 1 && dec[y].split[i] == 0) --i;
-            if (i == 1) {
-                if (nch < max_children) w.ch[nch++] = y;
-                else { atomicOr(err, 16u); break; }
-            } else {
-                const int k = dec[y].split[i];
-                if (sp + 2 > 16 || k < 1 || k >= i) { atomicOr(err, 16u); break; }
-                sn[sp] = nodes[y].right;
-                sb[sp++] = i - k;
-                sn[sp] = nodes[y].left;
-                sb[sp++] = k;
+    if (lane == 0) {
+        int32_t* ch = kids + group;
+        if (x < 0 || x > 2 * n - 2) {
+            atomicOr(err, 16u);
+        } else if (!wide_slot(dec, x)) {
+            ch[nch++] = x;                        // a root of at most 3 triangles
+        } else {
+            // expand (node, slots) pairs left to right, as DpCollapse::expand
+            int32_t sn[16];
+            int sb[16];
+            int sp = 0;
+            sn[sp] = nodes[x].right;
+            sb[sp++] = max_children - dec[x].wk;
+            sn[sp] = nodes[x].left;
+            sb[sp++] = dec[x].wk;
+            while (sp > 0) {
+                const int32_t y = sn[--sp];
+                int i = sb[sp];
+                if (y < 0 || y > 2 * n - 2 || i < 1 || i > max_children) { atomicOr(err, 16u); break; }
+                while (i > 1 && dec[y].split[i] == 0) --i;
+                if (i == 1) {
+                    if (nch < max_children) ch[nch++] = y;
+                    else { atomicOr(err, 16u); break; }
+                } else {
+                    const int k = dec[y].split[i];
+                    if (sp + 2 > 16 || k < 1 || k >= i) { atomicOr(err, 16u); break; }
+                    sn[sp] = nodes[y].right;
+                    sb[sp++] = i - k;
+                    sn[sp] = nodes[y].left;
+                    sb[sp++] = k;
+                }
             }
         }
     }
-    w.nch = nch;
-    GBox nb;
-    for (int k = 0; k < 3; ++k) { nb.lo[k] = FLT_MAX; nb.hi[k] = -FLT_MAX; }
-    for (int c = 0; c < nch; ++c) grow(nb, nodes[w.ch[c]].box);
-    float pc[3];
-    for (int k = 0; k < 3; ++k) pc[k] = 0.5f * (nb.lo[k] + nb.hi[k]);
-    bool used_slot[8] = {false, false, false, false, false, false, false, false};
-    bool placed[8] = {false, false, false, false, false, false, false, false};
+    nch = __shfl_sync(mask, nch, 0, 8);
+    __syncwarp(mask);
+    const bool used = (int)lane < nch;
+    const int32_t c = used ? kids[threadIdx.x] : -1;
+    GBox cb;
+    for (int k = 0; k < 3; ++k) { cb.lo[k] = FLT_MAX; cb.hi[k] = -FLT_MAX; }
+    uint32_t tris = 0;
+    bool wide = false;
+    if (used) {
+        cb = nodes[c].box;
+        wide = wide_slot(dec, c);
+        tris = wide ? 0u : nodes[c].count;
+    }
+    float dd[3];
+    for (int k = 0; k < 3; ++k) {
+        float lo = cb.lo[k], hi = cb.hi[k];
+        for (int o = 1; o < 8; o <<= 1) {
+            lo = fminf(lo, __shfl_xor_sync(mask, lo, o, 8));
+            hi = fmaxf(hi, __shfl_xor_sync(mask, hi, o, 8));
+        }
+        dd[k] = 0.5f * (cb.lo[k] + cb.hi[k]) - 0.5f * (lo + hi);
+    }
+    // greedy: the best (child, free slot) pair each round; ties to the lowest
+    // child, then the lowest slot
+    uint32_t taken = 0;
+    int slot = -1;
     for (int round = 0; round < nch; ++round) {
         float best = -FLT_MAX;
-        int bc = -1, bs = -1;
-        for (int c = 0; c < nch; ++c) {
-            if (placed[c]) continue;
-            const GBox& cb = nodes[w.ch[c]].box;
-            float dd[3];
-            for (int k = 0; k < 3; ++k) dd[k] = 0.5f * (cb.lo[k] + cb.hi[k]) - pc[k];
+        int bs = -1;
+        if (used && slot < 0)
             for (int s = 0; s < 8; ++s) {
-                if (used_slot[s]) continue;
+                if ((taken >> s) & 1u) continue;
                 const float sc = ((s & 1) ? dd[0] : -dd[0]) + ((s & 2) ? dd[1] : -dd[1]) + ((s & 4) ? dd[2] : -dd[2]);
-                if (sc > best) { best = sc; bc = c; bs = s; }
+                if (sc > best || bs < 0) { best = sc; bs = s; }
             }
+        float top = bs < 0 ? -FLT_MAX : best;
+        int who = bs < 0 ? 8 : (int)lane;
+        for (int o = 1; o < 8; o <<= 1) {
+            const float t = __shfl_xor_sync(mask, top, o, 8);
+            const int w = __shfl_xor_sync(mask, who, o, 8);
+            if (w < 8 && (who == 8 || t > top || (t == top && w < who))) { top = t; who = w; }
         }
-        placed[bc] = true;
-        used_slot[bs] = true;
-        w.slot_of[bc] = bs;
+        const int s = __shfl_sync(mask, bs, who & 7, 8);
+        taken |= 1u << (s & 7);
+        if ((int)lane == who) slot = s;
     }
-    uint32_t ni = 0, nt = 0;
-    for (int c = 0; c < nch; ++c) {
-        if (wide_slot(dec, w.ch[c])) ++ni;
-        else nt += nodes[w.ch[c]].count;
-    }
-    recs[f] = w;
-    cnt_int[f] = ni;
-    cnt_tri[f] = nt;
+    recs[f].child[lane] = -1;
+    __syncwarp(mask);
+    if (used && slot >= 0) recs[f].child[slot] = c;
+    uint64_t both = ((uint64_t)(wide ? 1u : 0u) << 32) | tris;
+    for (int o = 1; o < 8; o <<= 1) both += __shfl_xor_sync(mask, both, o, 8);
+    if (lane == 0) counts[f] = both;
 }
 
-// Encodes the wide nodes of one level (both device encodings), writes
-// the next level's frontier and the triangle records of the leaf slots.
-__global__ void k_emit(const GWide* __restrict__ recs, uint32_t F, uint32_t level_base, uint32_t next_base,
-                       uint32_t tri_level_base, const uint32_t* __restrict__ int_off,
-                       const uint32_t* __restrict__ tri_off, const GNode* __restrict__ nodes,
-                       const GDec* __restrict__ dec, const uint32_t* __restrict__ perm, const float* __restrict__ v1,
-                       const float* __restrict__ e1, const float* __restrict__ e2, DevNodeQ16* __restrict__ out,
-                       Bvh8FloatNode* __restrict__ fout, DevTriA* __restrict__ tris_a,
-                       DevTriB* __restrict__ tris_b, int32_t* __restrict__ next_front,
-                       uint32_t n_tris, uint32_t cap_nodes, uint32_t* err) {
-    const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= F) return;
-    if (level_base + f >= cap_nodes) {
-        atomicOr(err, 2u);
-        return;
+// The next level's frontier, in slot order, and the level's child and triangle
+// bases.
+__global__ void __launch_bounds__(kBlock) k_front(GWide* __restrict__ recs, uint32_t F, uint32_t next_base,
+                                                  uint32_t tri_level_base, const uint64_t* __restrict__ offsets,
+                                                  const GDec* __restrict__ dec, int32_t* __restrict__ next_front,
+                                                  uint32_t cap_nodes, uint32_t* err) {
+    const uint32_t f = (uint32_t)(((uint64_t)blockIdx.x * kBlock + threadIdx.x) >> 3);
+    const uint32_t lane = threadIdx.x & 7u;
+    if (f >= F) return;   // whole groups of 8
+    const uint32_t shift = threadIdx.x & 24u, mask = 0xFFu << shift;
+    const int32_t c = recs[f].child[lane];
+    const bool wide = c >= 0 && wide_slot(dec, c);
+    const uint32_t w = (__ballot_sync(mask, wide) >> shift) & 0xFFu;
+    const uint64_t off = offsets[f];
+    const uint32_t k = (uint32_t)(off >> 32) + __popc(w & ((1u << lane) - 1u));
+    if (wide) {
+        if (next_base + k < cap_nodes) next_front[k] = c;
+        else atomicOr(err, 2u);
     }
-    const GWide w = recs[f];
-    int child_at[8];
-    for (int s = 0; s < 8; ++s) child_at[s] = -1;
-    for (int c = 0; c < w.nch; ++c) child_at[w.slot_of[c]] = c;
-    GBox nb;
-    for (int k = 0; k < 3; ++k) { nb.lo[k] = FLT_MAX; nb.hi[k] = -FLT_MAX; }
-    for (int c = 0; c < w.nch; ++c) grow(nb, nodes[w.ch[c]].box);
-    DevNodeQ16 node;
-    memset(&node, 0, sizeof(node));
-    clear_planes16(node);
-    uint32_t slots = 0;
-    Bvh8FloatNode fnode;
-    memset(&fnode, 0, sizeof(fnode));
-    node.px = nb.lo[0];
-    node.py = nb.lo[1];
-    node.pz = nb.lo[2];
-    node.child_base = next_base + int_off[f];
-    node.tri_base = tri_level_base + tri_off[f];
-    uint32_t tri_o = 0, int_o = 0;
-    for (int s = 0; s < 8; ++s) {
-        const int c = child_at[s];
-        if (c < 0) {
-            for (int k = 0; k < 3; ++k) {
-                fnode.planes[k][0][s] = FLT_MAX;
-                fnode.planes[k][1][s] = -FLT_MAX;
-            }
+    if (lane == 0) {
+        recs[f].child_base = next_base + (uint32_t)(off >> 32);
+        recs[f].tri_base = tri_level_base + (uint32_t)off;
+    }
+}
+
+// Encodes the wide nodes (both device encodings) and writes the triangle
+// records of the leaf slots: 8 lanes per node, lane s for slot s.
+__global__ void __launch_bounds__(kBlock) k_emit(const GWide* __restrict__ recs, uint32_t N,
+                                                 const GNode* __restrict__ nodes, const GDec* __restrict__ dec,
+                                                 const uint32_t* __restrict__ perm, const float* __restrict__ v1,
+                                                 const float* __restrict__ e1, const float* __restrict__ e2,
+                                                 DevNodeQ16* __restrict__ out, Bvh8FloatNode* __restrict__ fout,
+                                                 DevTriA* __restrict__ tris_a, DevTriB* __restrict__ tris_b,
+                                                 uint32_t n_tris, uint32_t* err) {
+    const uint32_t f = (uint32_t)(((uint64_t)blockIdx.x * kBlock + threadIdx.x) >> 3);
+    const uint32_t s = threadIdx.x & 7u;
+    if (f >= N) return;   // whole groups of 8
+    const uint32_t mask = 0xFFu << (threadIdx.x & 24u);
+    const int32_t c = recs[f].child[s];
+    const uint32_t child_base = recs[f].child_base, tri_base = recs[f].tri_base;
+    GBox cb;
+    for (int k = 0; k < 3; ++k) { cb.lo[k] = FLT_MAX; cb.hi[k] = -FLT_MAX; }
+    uint32_t bits = 0, count = 0;
+    if (c >= 0) {
+        cb = nodes[c].box;
+        if (wide_slot(dec, c)) bits = 1u << s;
+        else {
+            count = min(nodes[c].count, kSlotTrisMax);
+            bits = ((1u << count) - 1u) << (8 + 3 * s);
+        }
+    }
+    const uint32_t slots = __reduce_or_sync(mask, bits);
+    float p[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        float lo = cb.lo[k];
+        for (int o = 1; o < 8; o <<= 1) lo = fminf(lo, __shfl_xor_sync(mask, lo, o, 8));
+        p[k] = lo;
+        fout[f].planes[k][0][s] = cb.lo[k];
+        fout[f].planes[k][1][s] = cb.hi[k];
+        // a word holds slots s and s + 4; an empty slot's planes are inverted
+        uint32_t l = 0x7F7Fu, h = 0xFF7Fu;
+        if (c >= 0) {
+            l = plane16((double)cb.lo[k] - (double)lo, false, s >= 4);
+            h = plane16((double)cb.hi[k] - (double)lo, true, s >= 4);
+        }
+        const uint32_t l4 = __shfl_xor_sync(mask, l, 4, 8), h4 = __shfl_xor_sync(mask, h, 4, 8);
+        if (s < 4) {
+            out[f].planes[k][0][s] = l | (l4 << 16);
+            out[f].planes[k][1][s] = h | (h4 << 16);
+        }
+    }
+    if (s == 0) {
+        out[f].px = p[0];
+        out[f].py = p[1];
+        out[f].pz = p[2];
+        out[f].child_base = fout[f].child_base = child_base;
+        out[f].tri_base = fout[f].tri_base = tri_base;
+        out[f].slots = fout[f].slots = slots;
+        out[f].pad[0] = out[f].pad[1] = fout[f].pad = 0;
+    }
+    out[f].pad2[s] = 0;
+    if (!count) return;
+    // the subtree's triangles, left to right (at most kSlotTrisMax)
+    uint32_t at = tri_base + __popc((slots >> 8) & ((1u << (3 * s)) - 1u)), found = 0;
+    int32_t stack[2 * kSlotTrisMax];
+    int sp = 0;
+    stack[sp++] = c;
+    while (sp > 0) {
+        const int32_t x = stack[--sp];
+        if (x < 0 || x > 2 * (int32_t)n_tris - 2) { atomicOr(err, 4u); break; }
+        const GNode& g = nodes[x];
+        if (g.left >= 0) {
+            if (sp + 2 > 2 * (int)kSlotTrisMax) { atomicOr(err, 4u); break; }
+            stack[sp++] = g.right;
+            stack[sp++] = g.left;
             continue;
         }
-        const GNode& cn = nodes[w.ch[c]];
-        for (int k = 0; k < 3; ++k) {
-            fnode.planes[k][0][s] = cn.box.lo[k];
-            fnode.planes[k][1][s] = cn.box.hi[k];
-            set_planes16(node, k, s, (double)cn.box.lo[k] - (double)nb.lo[k], (double)cn.box.hi[k] - (double)nb.lo[k]);
-        }
-        if (wide_slot(dec, w.ch[c])) {
-            slots |= 1u << s;
-            const uint32_t k = int_off[f] + int_o++;
-            if (next_base + k < cap_nodes) next_front[k] = w.ch[c];
-            else atomicOr(err, 2u);
-        } else {
-            slots |= ((1u << cn.count) - 1u) << (8 + 3 * s);
-            // the subtree's triangles, left to right (at most kSlotTrisMax)
-            uint32_t pos[kSlotTrisMax];
-            uint32_t np = 0;
-            int32_t stack[2 * kSlotTrisMax];
-            int sp = 0;
-            stack[sp++] = w.ch[c];
-            while (sp > 0) {
-                const int32_t x = stack[--sp];
-                if (x < 0 || x > 2 * (int32_t)n_tris - 2) { atomicOr(err, 4u); break; }
-                const GNode& g = nodes[x];
-                if (g.left < 0) {
-                    if (np < kSlotTrisMax) pos[np++] = g.first;
-                    else atomicOr(err, 4u);
-                } else if (sp + 2 <= 2 * (int)kSlotTrisMax) {
-                    stack[sp++] = g.right;
-                    stack[sp++] = g.left;
-                } else {
-                    atomicOr(err, 4u);
-                    break;
-                }
-            }
-            if (np != cn.count) atomicOr(err, 4u);
-            for (uint32_t i = 0; i < np; ++i) {
-                const uint32_t t = perm[pos[i]];
-                DevTriA ra;
-                for (int k = 0; k < 3; ++k) {
-                    ra.v1[k] = v1[3ull * t + k];
-                    ra.e1[k] = e1[3ull * t + k];
-                }
-                ra.face = t;
-                ra.e2x = e2[3ull * t];
-                if (node.tri_base + tri_o + i < n_tris) {
-                    tris_a[node.tri_base + tri_o + i] = ra;
-                    tris_b[node.tri_base + tri_o + i] = DevTriB{e2[3ull * t + 1], e2[3ull * t + 2]};
-                } else {
-                    atomicOr(err, 4u);
-                }
-            }
-            tri_o += np;
-        }
+        if (found == count || at >= n_tris) { atomicOr(err, 4u); break; }
+        const uint32_t t = perm[g.first];
+        tris_a[at] = DevTriA{{v1[3ull * t], v1[3ull * t + 1], v1[3ull * t + 2]}, t,
+                             {e1[3ull * t], e1[3ull * t + 1], e1[3ull * t + 2]}, e2[3ull * t]};
+        tris_b[at] = DevTriB{e2[3ull * t + 1], e2[3ull * t + 2]};
+        ++at;
+        ++found;
     }
-    node.slots = fnode.slots = slots;
-    out[level_base + f] = node;
-    fnode.child_base = node.child_base;
-    fnode.tri_base = node.tri_base;
-    fout[level_base + f] = fnode;
+    if (found != count) atomicOr(err, 4u);
 }
 
 uint32_t blocks(uint64_t n) { return (uint32_t)std::max<uint64_t>(1, (n + kBlock - 1) / kBlock); }
@@ -550,96 +693,96 @@ int build_bvh_gpu(const float* d_v1, const float* d_e1, const float* d_e2, uint3
                   uint32_t* max_depth, bool* fnodes_ok, cudaStream_t s) {
     if (n == 0) return set_error(CRT_ERR_INVALID, "scene has no triangles");
     if (n >= (1u << 30)) return set_error(CRT_ERR_LIMIT, "GPU BVH build: at most 2^30 triangles");
-    DevBuf maxbits, tbox, cent, cbounds, keys, vals, keys2, perm, gnodes, tmp, errbuf;
-    CRT_CUDA(errbuf.alloc(4));
-    CRT_CUDA(cudaMemsetAsync(errbuf.p, 0, 4, s));
-    uint32_t* err = errbuf.as<uint32_t>();
-    CRT_CUDA(maxbits.alloc(4));
-    CRT_CUDA(cudaMemsetAsync(maxbits.p, 0, 4, s));
-    k_max_abs<<<blocks(3ull * n) < 1024 ? blocks(3ull * n) : 1024, kBlock, 0, s>>>(d_v1, d_e1, d_e2, 3 * n,
-                                                                                  maxbits.as<uint32_t>());
+    const int ni = (int)n;
+    const size_t n1 = n, nn2 = 2 * n1 - 1;
+    size_t sort_bytes = 0, scan_bytes = 0;
+    CRT_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, (const uint64_t*)nullptr, (uint64_t*)nullptr,
+                                             (const uint32_t*)nullptr, (uint32_t*)nullptr, ni, 0, 63, s));
+    CRT_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, (const uint64_t*)nullptr, (uint64_t*)nullptr, ni + 1, s));
+    // One allocation for every temporary.  The first part serves in turn the
+    // boxes and sort keys, the collapse's costs, and the collapse's levels.
+    Arena mem;
+    const size_t phase0 = mem.at;
+    const size_t o_tbox = mem.take(n1 * sizeof(GBox)), o_cent = mem.take(n1 * 12), o_keys = mem.take(n1 * 8),
+                 o_vals = mem.take(n1 * 4), o_keys2 = mem.take(n1 * 8), o_sort = mem.take(sort_bytes);
+    size_t end = mem.at;
+    mem.at = phase0;
+    const size_t o_cost = mem.take(nn2 * 8 * sizeof(float));
+    end = std::max(end, mem.at);
+    mem.at = phase0;
+    const size_t o_recs = mem.take(n1 * sizeof(GWide)), o_cnt = mem.take((n1 + 1) * 8), o_off = mem.take((n1 + 1) * 8),
+                 o_fa = mem.take(n1 * 4), o_fb = mem.take(n1 * 4), o_scan = mem.take(scan_bytes);
+    mem.at = std::max(end, mem.at);
+    const size_t o_perm = mem.take(n1 * 4), o_nodes = mem.take(nn2 * sizeof(GNode)), o_ca = mem.take(n1 * 4),
+                 o_cb = mem.take(n1 * 4), o_pair = mem.take(n1 * 4), o_counts = mem.take((n1 / kBlock + 1) * 8),
+                 o_dec = mem.take(nn2 * sizeof(GDec)), o_flags = mem.take(n1 * 4), o_small = mem.take(64);
+    DevBuf arena;
+    CRT_CUDA(arena.alloc(mem.at));
+    char* base = arena.as<char>();
+    uint32_t* err = reinterpret_cast<uint32_t*>(base + o_small);       // word 0: error bits, 1: largest magnitude
+    uint32_t* cbounds = err + 2;                                       // words 2-7: centroid bounds
+    PlocState* ploc = reinterpret_cast<PlocState*>(base + o_small + 32);
+    const uint32_t init[8] = {0u, 0u, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u};
+    CRT_CUDA(cudaMemcpyAsync(err, init, sizeof(init), cudaMemcpyHostToDevice, s));
+    k_max_abs<<<blocks(3ull * n) < 1024 ? blocks(3ull * n) : 1024, kBlock, 0, s>>>(d_v1, d_e1, d_e2, 3 * n, err + 1);
     uint32_t mb = 0;
-    CRT_CUDA(cudaMemcpyAsync(&mb, maxbits.p, 4, cudaMemcpyDeviceToHost, s));
+    CRT_CUDA(cudaMemcpyAsync(&mb, err + 1, 4, cudaMemcpyDeviceToHost, s));
     CRT_CUDA(cudaStreamSynchronize(s));
     float maxabs;
     std::memcpy(&maxabs, &mb, 4);
     const float margin = (float)std::ldexp(std::max(1.0, (double)maxabs), -15);
 
-    CRT_CUDA(tbox.alloc((size_t)n * sizeof(GBox)));
-    CRT_CUDA(cent.alloc((size_t)n * 12));
-    CRT_CUDA(cbounds.alloc(24));
-    const uint32_t init[6] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u};
-    CRT_CUDA(cudaMemcpyAsync(cbounds.p, init, 24, cudaMemcpyHostToDevice, s));
-    k_tri_boxes<<<std::min<uint32_t>(blocks(n), 4096), kBlock, 0, s>>>(d_v1, d_e1, d_e2, n, margin, tbox.as<GBox>(),
-                                                                        cent.as<float>(), cbounds.as<uint32_t>());
-    CRT_CUDA(keys.alloc((size_t)n * 8));
-    CRT_CUDA(vals.alloc((size_t)n * 4));
-    CRT_CUDA(keys2.alloc((size_t)n * 8));
-    CRT_CUDA(perm.alloc((size_t)n * 4));
-    k_morton<<<std::min<uint32_t>(blocks(n), 4096), kBlock, 0, s>>>(cent.as<float>(), n, cbounds.as<uint32_t>(),
-                                                                     keys.as<uint64_t>(), vals.as<uint32_t>());
-    size_t tmp_bytes = 0;
-    CRT_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys.as<uint64_t>(), keys2.as<uint64_t>(),
-                                             vals.as<uint32_t>(), perm.as<uint32_t>(), (int)n, 0, 63, s));
-    CRT_CUDA(tmp.alloc(tmp_bytes));
-    CRT_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tmp_bytes, keys.as<uint64_t>(), keys2.as<uint64_t>(),
-                                             vals.as<uint32_t>(), perm.as<uint32_t>(), (int)n, 0, 63, s));
-    const int ni = (int)n;
-    CRT_CUDA(gnodes.alloc((size_t)(2 * n - 1) * sizeof(GNode)));
-    CRT_CUDA(cudaMemsetAsync(gnodes.p, 0xFF, gnodes.bytes, s));   // every parent / child index starts at -1
-    GNode* gn = gnodes.as<GNode>();
-    k_leaves<<<blocks(n), kBlock, 0, s>>>(tbox.as<GBox>(), perm.as<uint32_t>(), ni, gn);
-    int32_t root = (int32_t)n - 1;   // a lone triangle is its own root
+    GBox* tbox = reinterpret_cast<GBox*>(base + o_tbox);
+    float* cent = reinterpret_cast<float*>(base + o_cent);
+    uint64_t* keys = reinterpret_cast<uint64_t*>(base + o_keys);
+    uint64_t* keys2 = reinterpret_cast<uint64_t*>(base + o_keys2);
+    uint32_t* vals = reinterpret_cast<uint32_t*>(base + o_vals);
+    uint32_t* perm = reinterpret_cast<uint32_t*>(base + o_perm);
+    k_tri_boxes<<<std::min<uint32_t>(blocks(n), 1216), kBlock, 0, s>>>(d_v1, d_e1, d_e2, n, margin, tbox, cent, cbounds);
+    k_morton<<<std::min<uint32_t>(blocks(n), 4096), kBlock, 0, s>>>(cent, n, cbounds, keys, vals);
+    CRT_CUDA(cub::DeviceRadixSort::SortPairs(base + o_sort, sort_bytes, keys, keys2, vals, perm, ni, 0, 63, s));
+    GNode* gn = reinterpret_cast<GNode*>(base + o_nodes);
+    k_leaves<<<blocks(n), kBlock, 0, s>>>(tbox, perm, ni, gn);
+    int32_t root = ni - 1;   // a lone triangle is its own root
     if (n > 1) {
-        // PLOC iterations over the cluster list (Morton order), ping-ponged
-        DevBuf cl_a, cl_b, nnb, fl, scan, ploc_tmp;
-        CRT_CUDA(cl_a.alloc((size_t)n * 4));
-        CRT_CUDA(cl_b.alloc((size_t)n * 4));
-        CRT_CUDA(nnb.alloc((size_t)n * 4));
-        CRT_CUDA(fl.alloc((size_t)(n + 1) * 8));
-        CRT_CUDA(scan.alloc((size_t)(n + 1) * 8));
-        k_ploc_init<<<blocks(n), kBlock, 0, s>>>(cl_a.as<int32_t>(), ni);
-        size_t ploc_bytes = 0;
-        CRT_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, ploc_bytes, fl.as<uint64_t>(), scan.as<uint64_t>(),
-                                               (int)n + 1, s));
-        CRT_CUDA(ploc_tmp.alloc(ploc_bytes));
-        int32_t* cur = cl_a.as<int32_t>();
-        int32_t* nxt = cl_b.as<int32_t>();
-        uint32_t m = n;
-        int32_t next_id = (int32_t)n - 2;
-        for (uint32_t iter = 0; m > 1; ++iter) {
-            if (iter >= n) return set_error(CRT_ERR_CUDA, "GPU BVH build: clustering did not converge");
-            k_ploc_nn<<<blocks(m), kBlock, 0, s>>>(cur, (int)m, gn, nnb.as<int32_t>(), ni, err);
-            k_ploc_flags<<<blocks(m), kBlock, 0, s>>>(nnb.as<int32_t>(), (int)m, fl.as<uint64_t>());
-            CRT_CUDA(cudaMemsetAsync(fl.as<uint64_t>() + m, 0, 8, s));
-            CRT_CUDA(cub::DeviceScan::ExclusiveSum(ploc_tmp.p, ploc_bytes, fl.as<uint64_t>(), scan.as<uint64_t>(),
-                                                   (int)m + 1, s));
-            k_ploc_merge<<<blocks(m), kBlock, 0, s>>>(cur, nnb.as<int32_t>(), (int)m, scan.as<uint64_t>(), next_id,
-                                                      gn, nxt, ni, err);
-            uint64_t total = 0;
-            CRT_CUDA(cudaMemcpyAsync(&total, scan.as<uint64_t>() + m, 8, cudaMemcpyDeviceToHost, s));
+        // PLOC iterations over the cluster list (Morton order), ping-ponged.
+        // The list's length stays on the device; the host reads it after every
+        // few iterations, to shrink the grid and to end.  (Neighbours, flags, a
+        // library scan, the merge and a host read each iteration: 2.6 ms of 2.17M
+        // triangles' build; three kernels and a read every fourth: 1.1.)
+        constexpr int kPerSync = 4;
+        int32_t* cur = reinterpret_cast<int32_t*>(base + o_ca);
+        int32_t* nxt = reinterpret_cast<int32_t*>(base + o_cb);
+        int32_t* pair = reinterpret_cast<int32_t*>(base + o_pair);
+        uint64_t* counts = reinterpret_cast<uint64_t*>(base + o_counts);
+        k_ploc_init<<<blocks(n), kBlock, 0, s>>>(cur, ni, ploc);
+        PlocState at{ni, ni - 2};
+        for (uint32_t iter = 0; at.m > 1;) {
+            const int32_t before = at.m;
+            for (int k = 0; k < kPerSync; ++k, ++iter) {
+                const PlocState* st = ploc + (iter & 1u);
+                k_ploc_pairs<<<blocks(before), kBlock, 0, s>>>(cur, st, gn, pair, counts, ni, err);
+                k_ploc_scan<<<1, 1024, 0, s>>>(counts, st, ploc + ((iter + 1u) & 1u), err);
+                k_ploc_merge<<<blocks(before), kBlock, 0, s>>>(cur, pair, st, counts, gn, nxt, ni, err);
+                std::swap(cur, nxt);
+            }
+            uint32_t e = 0;
+            CRT_CUDA(cudaMemcpyAsync(&at, ploc + (iter & 1u), sizeof(at), cudaMemcpyDeviceToHost, s));
+            CRT_CUDA(cudaMemcpyAsync(&e, err, 4, cudaMemcpyDeviceToHost, s));
             CRT_CUDA(cudaStreamSynchronize(s));
-            const uint32_t survivors = (uint32_t)(total >> 32), merges = (uint32_t)(total & 0xFFFFFFFFull);
-            if (merges == 0 || survivors + merges != m || (int64_t)next_id + 1 < (int64_t)merges)
+            if (e || at.m < 1 || at.m >= before)
                 return set_error(CRT_ERR_CUDA, "GPU BVH build: inconsistent clustering step");
-            m = survivors;
-            next_id -= (int32_t)merges;
-            std::swap(cur, nxt);
         }
         CRT_CUDA(cudaMemcpyAsync(&root, cur, 4, cudaMemcpyDeviceToHost, s));
         CRT_CUDA(cudaStreamSynchronize(s));
-        if (root != 0 || next_id != -1) return set_error(CRT_ERR_CUDA, "GPU BVH build: clustering left no single root");
+        if (root != 0 || at.next_id != -1) return set_error(CRT_ERR_CUDA, "GPU BVH build: clustering left no single root");
     }
     // the collapse's costs and decisions, bottom-up
-    DevBuf dp_cost, dp_dec, dp_flags;
-    CRT_CUDA(dp_cost.alloc((size_t)(2 * n - 1) * 8 * sizeof(float)));
-    CRT_CUDA(dp_dec.alloc((size_t)(2 * n - 1) * sizeof(GDec)));
-    CRT_CUDA(dp_flags.alloc((size_t)n * 4));
-    CRT_CUDA(cudaMemsetAsync(dp_flags.p, 0, (size_t)n * 4, s));
-    k_dp_leaves<<<blocks(n), kBlock, 0, s>>>(ni, gn, max_children, dp_cost.as<float>(), dp_dec.as<GDec>());
-    k_dp_up<<<blocks(n), kBlock, 0, s>>>(ni, gn, max_children, dp_cost.as<float>(), dp_dec.as<GDec>(),
-                                         dp_flags.as<uint32_t>(), err);
-    const GDec* dec = dp_dec.as<GDec>();
+    float* cost = reinterpret_cast<float*>(base + o_cost);
+    GDec* dec = reinterpret_cast<GDec*>(base + o_dec);
+    uint32_t* flags = reinterpret_cast<uint32_t*>(base + o_flags);
+    CRT_CUDA(cudaMemsetAsync(flags, 0, n1 * 4, s));
+    (max_children == 4 ? k_dp_up<4> : k_dp_up<8>)<<<blocks(n), kBlock, 0, s>>>(ni, gn, cost, dec, flags, err);
     CRT_CUDA(cudaGetLastError());
     {   // the collapse follows child links: stop here if any were not set
         uint32_t e = 0;
@@ -648,60 +791,49 @@ int build_bvh_gpu(const float* d_v1, const float* d_e1, const float* d_e2, uint3
         if (e) return set_error(CRT_ERR_CUDA, "GPU BVH build: inconsistent hierarchy (" + std::to_string(e) + ")");
     }
 
-    // ---- collapse level by level -------------------------------------------
+    // ---- collapse level by level, then encode all nodes at once ------------
     const uint32_t cap_nodes = n;   // a wide node holds >= 1 triangle of its own subtree
-    CRT_CUDA(nodes_out.alloc((size_t)cap_nodes * sizeof(DevNodeQ16)));
-    CRT_CUDA(fnodes_out.alloc((size_t)cap_nodes * sizeof(Bvh8FloatNode)));
-    CRT_CUDA(tris_out.alloc((size_t)n * (sizeof(DevTriA) + sizeof(DevTriB))));
-    DevBuf front_a, front_b, recs, cnt_int, cnt_tri, off_int, off_tri, scan_tmp;
-    CRT_CUDA(front_a.alloc((size_t)cap_nodes * 4));
-    CRT_CUDA(front_b.alloc((size_t)cap_nodes * 4));
-    CRT_CUDA(recs.alloc((size_t)cap_nodes * sizeof(GWide)));
-    CRT_CUDA(cnt_int.alloc((size_t)cap_nodes * 4 + 4));
-    CRT_CUDA(cnt_tri.alloc((size_t)cap_nodes * 4 + 4));
-    CRT_CUDA(off_int.alloc((size_t)cap_nodes * 4 + 4));
-    CRT_CUDA(off_tri.alloc((size_t)cap_nodes * 4 + 4));
-    size_t scan_bytes = 0;
-    CRT_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, cnt_int.as<uint32_t>(), off_int.as<uint32_t>(),
-                                           (int)cap_nodes + 1, s));
-    CRT_CUDA(scan_tmp.alloc(scan_bytes));
-    CRT_CUDA(cudaMemcpyAsync(front_a.p, &root, 4, cudaMemcpyHostToDevice, s));
+    GWide* recs = reinterpret_cast<GWide*>(base + o_recs);
+    uint64_t* cnt = reinterpret_cast<uint64_t*>(base + o_cnt);
+    uint64_t* off = reinterpret_cast<uint64_t*>(base + o_off);
+    int32_t* cur = reinterpret_cast<int32_t*>(base + o_fa);
+    int32_t* nxt = reinterpret_cast<int32_t*>(base + o_fb);
+    CRT_CUDA(cudaMemcpyAsync(cur, &root, 4, cudaMemcpyHostToDevice, s));
     uint32_t F = 1, level_base = 0, tri_base = 0, depth = 0;
-    int32_t* cur = front_a.as<int32_t>();
-    int32_t* nxt = front_b.as<int32_t>();
     while (F > 0) {
         if (++depth > max_levels) return set_error(CRT_ERR_LIMIT, "BVH deeper than the traversal stack allows");
-        k_choose<<<blocks(F), kBlock, 0, s>>>(cur, F, gn, dec, max_children, recs.as<GWide>(), cnt_int.as<uint32_t>(),
-                                              cnt_tri.as<uint32_t>(), ni, err);
-        // exclusive sums over F + 1 entries: the last is each level's total
-        CRT_CUDA(cudaMemsetAsync(cnt_int.as<uint32_t>() + F, 0, 4, s));
-        CRT_CUDA(cudaMemsetAsync(cnt_tri.as<uint32_t>() + F, 0, 4, s));
-        CRT_CUDA(cub::DeviceScan::ExclusiveSum(scan_tmp.p, scan_bytes, cnt_int.as<uint32_t>(), off_int.as<uint32_t>(),
-                                               (int)F + 1, s));
-        CRT_CUDA(cub::DeviceScan::ExclusiveSum(scan_tmp.p, scan_bytes, cnt_tri.as<uint32_t>(), off_tri.as<uint32_t>(),
-                                               (int)F + 1, s));
+        k_choose<<<blocks(8ull * F), kBlock, 0, s>>>(cur, F, gn, dec, max_children, recs + level_base, cnt, ni, err);
+        // exclusive sums over F + 1 entries: the last is the level's totals
+        CRT_CUDA(cudaMemsetAsync(cnt + F, 0, 8, s));
+        CRT_CUDA(cub::DeviceScan::ExclusiveSum(base + o_scan, scan_bytes, cnt, off, (int)F + 1, s));
         const uint32_t next_base = level_base + F;
-        k_emit<<<blocks(F), kBlock, 0, s>>>(recs.as<GWide>(), F, level_base, next_base, tri_base,
-                                            off_int.as<uint32_t>(), off_tri.as<uint32_t>(), gn, dec, perm.as<uint32_t>(),
-                                            d_v1, d_e1, d_e2, nodes_out.as<DevNodeQ16>(), fnodes_out.as<Bvh8FloatNode>(),
-                                            tris_out.as<DevTriA>(),
-                                            reinterpret_cast<DevTriB*>(tris_out.as<DevTriA>() + n), nxt, n, cap_nodes, err);
-        uint32_t totals[2];
-        CRT_CUDA(cudaMemcpyAsync(&totals[0], off_int.as<uint32_t>() + F, 4, cudaMemcpyDeviceToHost, s));
-        CRT_CUDA(cudaMemcpyAsync(&totals[1], off_tri.as<uint32_t>() + F, 4, cudaMemcpyDeviceToHost, s));
+        k_front<<<blocks(8ull * F), kBlock, 0, s>>>(recs + level_base, F, next_base, tri_base, off, dec, nxt,
+                                                    cap_nodes, err);
+        uint64_t totals = 0;
+        uint32_t e = 0;
+        CRT_CUDA(cudaMemcpyAsync(&totals, off + F, 8, cudaMemcpyDeviceToHost, s));
+        CRT_CUDA(cudaMemcpyAsync(&e, err, 4, cudaMemcpyDeviceToHost, s));
         CRT_CUDA(cudaStreamSynchronize(s));
         CRT_CUDA(cudaGetLastError());
+        if (e) return set_error(CRT_ERR_CUDA, "GPU BVH build: inconsistent tree (" + std::to_string(e) + ")");
         level_base = next_base;
-        tri_base += totals[1];
-        F = totals[0];
-        if (level_base + F > cap_nodes) return set_error(CRT_ERR_LIMIT, "GPU BVH node count overflow");
+        tri_base += (uint32_t)totals;
+        F = (uint32_t)(totals >> 32);
+        if ((uint64_t)level_base + F > cap_nodes) return set_error(CRT_ERR_LIMIT, "GPU BVH node count overflow");
         std::swap(cur, nxt);
     }
+    if (tri_base != n) return set_error(CRT_ERR_CUDA, "GPU BVH lost triangles");
+    CRT_CUDA(nodes_out.alloc((size_t)level_base * sizeof(DevNodeQ16)));
+    CRT_CUDA(fnodes_out.alloc((size_t)level_base * sizeof(Bvh8FloatNode)));
+    CRT_CUDA(tris_out.alloc(n1 * (sizeof(DevTriA) + sizeof(DevTriB))));
+    k_emit<<<blocks(8ull * level_base), kBlock, 0, s>>>(
+        recs, level_base, gn, dec, perm, d_v1, d_e1, d_e2, nodes_out.as<DevNodeQ16>(), fnodes_out.as<Bvh8FloatNode>(),
+        tris_out.as<DevTriA>(), reinterpret_cast<DevTriB*>(tris_out.as<DevTriA>() + n), n, err);
     uint32_t errbits = 0;
     CRT_CUDA(cudaMemcpyAsync(&errbits, err, 4, cudaMemcpyDeviceToHost, s));
     CRT_CUDA(cudaStreamSynchronize(s));
+    CRT_CUDA(cudaGetLastError());
     if (errbits) return set_error(CRT_ERR_CUDA, "GPU BVH build: inconsistent tree (" + std::to_string(errbits) + ")");
-    if (tri_base != n) return set_error(CRT_ERR_CUDA, "GPU BVH lost triangles");
     *num_nodes = level_base;
     *max_depth = depth;
     *fnodes_ok = level_base <= (1u << 24);

@@ -25,6 +25,16 @@ int cuda_error(cudaError_t e, const char* what);
         if (e_ != cudaSuccess) return cuda_error(e_, #call); \
     } while (0)
 
+// Offsets of 256-byte aligned parts of one allocation.
+struct Arena {
+    size_t at = 0;
+    size_t take(size_t bytes) {
+        const size_t here = at;
+        at += (bytes + 255) & ~(size_t)255;
+        return here;
+    }
+};
+
 // Owning device buffer.
 struct DevBuf {
     void* p = nullptr;

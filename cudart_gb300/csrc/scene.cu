@@ -148,13 +148,19 @@ static int install_bvh(crt_scene s, Bvh8& b, uint32_t width) {
     DevBuf nodes, fnodes, tris;
     int st = CRT_OK;
     if (b.fnodes_ok && (st = upload(fnodes, b.fnodes))) return st;
-    DevBuf raw_nodes, raw_tris;
-    if ((st = upload(raw_nodes, b.nodes)) || (st = upload(raw_tris, b.tris))) return st;
     const uint32_t nn = (uint32_t)b.nodes.size(), nt = (uint32_t)b.tris.size();
+    Arena mem;
+    const size_t o_nodes = mem.take(nn * sizeof(Bvh8Node)), o_tris = mem.take((size_t)nt * sizeof(TriRecord));
+    DevBuf raw;
+    CRT_CUDA(raw.alloc(mem.at));
+    const Bvh8Node* raw_nodes = reinterpret_cast<Bvh8Node*>(raw.as<char>() + o_nodes);
+    const TriRecord* raw_tris = reinterpret_cast<TriRecord*>(raw.as<char>() + o_tris);
+    CRT_CUDA(cudaMemcpy((void*)raw_nodes, b.nodes.data(), nn * sizeof(Bvh8Node), cudaMemcpyHostToDevice));
+    CRT_CUDA(cudaMemcpy((void*)raw_tris, b.tris.data(), (size_t)nt * sizeof(TriRecord), cudaMemcpyHostToDevice));
     CRT_CUDA(nodes.alloc((size_t)nn * sizeof(DevNodeQ16)));
     CRT_CUDA(tris.alloc((size_t)nt * (sizeof(DevTriA) + sizeof(DevTriB))));
     k_pack_bvh<<<(uint32_t)std::min<uint64_t>(((uint64_t)std::max(nn, nt) + 255) / 256, 4096), 256>>>(
-        raw_nodes.as<Bvh8Node>(), b.fnodes_ok ? fnodes.as<Bvh8FloatNode>() : nullptr, nn, raw_tris.as<TriRecord>(), nt, nodes.as<DevNodeQ16>(), tris.as<DevTriA>(),
+        raw_nodes, b.fnodes_ok ? fnodes.as<Bvh8FloatNode>() : nullptr, nn, raw_tris, nt, nodes.as<DevNodeQ16>(), tris.as<DevTriA>(),
         reinterpret_cast<DevTriB*>(tris.as<DevTriA>() + nt));
     CRT_CUDA(cudaGetLastError());
     CRT_CUDA(cudaDeviceSynchronize());
@@ -389,9 +395,12 @@ int crt_scene_create(const crt_scene_desc* d, crt_scene* out) {
     if (d->num_materials == 0 || !d->materials)
         return set_error(CRT_ERR_INVALID, "scene has no materials");
     if (n >= (1u << 31)) return set_error(CRT_ERR_LIMIT, "more than 2^31 triangles");
-    for (uint32_t i = 0; i < n; ++i)
-        if (d->material_ids[i] >= d->num_materials)
-            return set_error(CRT_ERR_INVALID, "material id out of range at face " + std::to_string(i));
+    uint32_t top_id = 0;   // a plain maximum vectorises; the offender is looked up only if there is one
+    for (uint32_t i = 0; i < n; ++i) top_id = std::max(top_id, d->material_ids[i]);
+    if (top_id >= d->num_materials)
+        for (uint32_t i = 0; i < n; ++i)
+            if (d->material_ids[i] >= d->num_materials)
+                return set_error(CRT_ERR_INVALID, "material id out of range at face " + std::to_string(i));
     for (uint32_t m = 0; m < d->num_materials; ++m) {
         int t = d->materials[m].texture;
         if (t != CRT_NO_TEXTURE && (t < 0 || (uint32_t)t >= d->num_textures))
@@ -420,8 +429,17 @@ int crt_scene_create(const crt_scene_desc* d, crt_scene* out) {
             s->lights.push_back(d->light_indices[i]);
         }
     } else {
-        for (uint32_t i = 0; i < n; ++i)
-            if (d->materials[d->material_ids[i]].bsdf == CRT_BSDF_EMISSIVE) s->lights.push_back(i);
+        // emitters are few: a byte per material, tested by the block
+        std::vector<uint8_t> emits(d->num_materials);
+        for (uint32_t m = 0; m < d->num_materials; ++m) emits[m] = d->materials[m].bsdf == CRT_BSDF_EMISSIVE;
+        for (uint32_t i0 = 0; i0 < n; i0 += 64) {
+            const uint32_t i1 = std::min(n, i0 + 64);
+            uint32_t any = 0;
+            for (uint32_t i = i0; i < i1; ++i) any |= emits[d->material_ids[i]];
+            if (!any) continue;
+            for (uint32_t i = i0; i < i1; ++i)
+                if (emits[d->material_ids[i]]) s->lights.push_back(i);
+        }
     }
     if (s->lights.empty()) {
         delete s;
@@ -470,43 +488,49 @@ int crt_scene_create(const crt_scene_desc* d, crt_scene* out) {
     // shading and uv records there.
     int st = CRT_OK;
     {
-        DevBuf dpos, dnor, duv, dmid, dv1, de1, de2;
-        if ((st = upload_raw(dpos, d->positions, 9ull * n)) || (st = upload_raw(dnor, d->normals, 9ull * n)) ||
-            (d->uvs && (st = upload_raw(duv, d->uvs, 6ull * n))) || (st = upload_raw(dmid, d->material_ids, n))) {
-            delete s;
-            return st;
-        }
-        DevBuf dbad;
-        cudaError_t e = dbad.alloc(4);
-        if (e == cudaSuccess) e = cudaMemset(dbad.p, 0xFF, 4);   // lowest bad face, or UINT32_MAX
-        if (e == cudaSuccess) e = dv1.alloc(12ull * n);
-        if (e == cudaSuccess) e = de1.alloc(12ull * n);
-        if (e == cudaSuccess) e = de2.alloc(12ull * n);
+        // (one allocation for what the caller's arrays and the edges need here)
+        Arena mem;
+        const size_t o_pos = mem.take(36ull * n), o_nor = mem.take(36ull * n), o_uv = mem.take(d->uvs ? 24ull * n : 0),
+                     o_mid = mem.take(4ull * n), o_v1 = mem.take(12ull * n), o_e1 = mem.take(12ull * n),
+                     o_e2 = mem.take(12ull * n), o_bad = mem.take(4);
+        DevBuf temp;
+        cudaError_t e = temp.alloc(mem.at);
         if (e == cudaSuccess) e = s->shade.alloc(48ull * n);
         if (e == cudaSuccess) e = s->uvs.alloc(32ull * n);
         if (e != cudaSuccess) { delete s; return cuda_error(e, "cudaMalloc"); }
-        const uint32_t grid = (uint32_t)std::min<uint64_t>((n + 255) / 256, 4096);
-        k_pack_faces<<<grid, 256>>>(dpos.as<float>(), dnor.as<float>(), d->uvs ? duv.as<float>() : nullptr,
-                                    dmid.as<uint32_t>(), n, (d->flags & CRT_SCENE_EDGES) != 0, dv1.as<float>(),
-                                    de1.as<float>(), de2.as<float>(), s->shade.as<float4>(), s->uvs.as<float4>(),
-                                    dbad.as<uint32_t>());
+        char* base = temp.as<char>();
+        float* v1 = reinterpret_cast<float*>(base + o_v1);
+        float* e1 = reinterpret_cast<float*>(base + o_e1);
+        float* e2 = reinterpret_cast<float*>(base + o_e2);
+        uint32_t* bad = reinterpret_cast<uint32_t*>(base + o_bad);
+        e = cudaMemcpy(base + o_pos, d->positions, 36ull * n, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMemcpy(base + o_nor, d->normals, 36ull * n, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess && d->uvs) e = cudaMemcpy(base + o_uv, d->uvs, 24ull * n, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMemcpy(base + o_mid, d->material_ids, 4ull * n, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMemset(bad, 0xFF, 4);   // lowest bad face, or UINT32_MAX
+        if (e != cudaSuccess) { delete s; return cuda_error(e, "cudaMemcpy"); }
+        const uint32_t grid = (uint32_t)std::min<uint64_t>((n + 255ull) / 256, 4096);
+        k_pack_faces<<<grid, 256>>>(reinterpret_cast<float*>(base + o_pos), reinterpret_cast<float*>(base + o_nor),
+                                    d->uvs ? reinterpret_cast<float*>(base + o_uv) : nullptr,
+                                    reinterpret_cast<uint32_t*>(base + o_mid), n, (d->flags & CRT_SCENE_EDGES) != 0, v1, e1,
+                                    e2, s->shade.as<float4>(), s->uvs.as<float4>(), bad);
         e = cudaGetLastError();
         uint32_t bad_face = UINT32_MAX;
-        if (e == cudaSuccess) e = cudaMemcpy(&bad_face, dbad.p, 4, cudaMemcpyDeviceToHost);
+        if (e == cudaSuccess) e = cudaMemcpy(&bad_face, bad, 4, cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) { delete s; return cuda_error(e, "k_pack_faces"); }
         if (bad_face != UINT32_MAX) {
             delete s;
             return set_error(CRT_ERR_INVALID, "non-finite vertex coordinate in face " + std::to_string(bad_face));
         }
         if (s->builder == CRT_BVH_GPU) {
-            st = build_on_device(s, dv1.as<float>(), de1.as<float>(), de2.as<float>(), n, width);
+            st = build_on_device(s, v1, e1, e2, n, width);
         } else {
-            std::vector<float> v1(3ull * n), e1(3ull * n), e2(3ull * n);
-            e = cudaMemcpy(v1.data(), dv1.p, 12ull * n, cudaMemcpyDeviceToHost);
-            if (e == cudaSuccess) e = cudaMemcpy(e1.data(), de1.p, 12ull * n, cudaMemcpyDeviceToHost);
-            if (e == cudaSuccess) e = cudaMemcpy(e2.data(), de2.p, 12ull * n, cudaMemcpyDeviceToHost);
+            std::vector<float> hv1(3ull * n), he1(3ull * n), he2(3ull * n);
+            e = cudaMemcpy(hv1.data(), v1, 12ull * n, cudaMemcpyDeviceToHost);
+            if (e == cudaSuccess) e = cudaMemcpy(he1.data(), e1, 12ull * n, cudaMemcpyDeviceToHost);
+            if (e == cudaSuccess) e = cudaMemcpy(he2.data(), e2, 12ull * n, cudaMemcpyDeviceToHost);
             if (e != cudaSuccess) { delete s; return cuda_error(e, "cudaMemcpy"); }
-            st = build_and_install(s, v1, e1, e2, n, width);
+            st = build_and_install(s, hv1, he1, he2, n, width);
         }
         if (st != CRT_OK) { delete s; return st; }
     }
