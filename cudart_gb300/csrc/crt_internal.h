@@ -83,6 +83,8 @@ struct WaveBuffers {
     bool octant = false;            // queues hold 8 octant regions
     crt::DevBuf ray_o, color, hit, queue_a, queue_b, shadow, shadow_q, counters, waves, segs, prof;
     crt::DevBuf adj_L, adj_W, adj_shadow, adj_hist;   // adjoint replay state, allocated on first use
+    crt::DevBuf adj_hits, adj_vis;                    // the primal trace's record (wavefront.cu)
+    bool adj_no_room = false;                         // no memory for the record
 };
 
 // One independent set of wavefront buffers with its own stream and captured
@@ -92,8 +94,8 @@ struct WaveSet {
     cudaStream_t stream = nullptr;
     cudaEvent_t acc_done = nullptr;   // recorded after this set's latest accumulate
     void* graph = nullptr;
-    void* adj_graph = nullptr;        // adjoint wave body, captured for adj_key's pointers
-    const void* adj_key[3] = {nullptr, nullptr, nullptr};
+    void* adj_graph = nullptr;        // adjoint wave body, captured for adj_key's pixel weights
+    const void* adj_key = nullptr;
     uint32_t adj_flags = 0;
 };
 
@@ -131,6 +133,7 @@ struct crt_render_s {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     crt::DevBuf accum, lut, ray_counts, view_table, staging;
+    crt::DevBuf adj_grad;           // gradient sums of an adjoint pass
     crt::DevBuf path_color;         // radiance per path of a pass on the path kernel
     std::vector<WaveSet> sets;
     uint32_t scene_generation = 0;  // scene BVH the captured wave graphs point at

@@ -152,11 +152,12 @@ struct WaveParams {
     float4* st_L;               // radiance of each path's primal trace
     float4* st_W;               // adjoint weight of each path's pixel
     float4* shd_grad;           // per shadow request: w * d contrib / d ka, light material
-    float* grad_kd;             // [n_mats][3], added to
-    float* grad_ka;             // [n_mats][3], added to
+    double* grad;               // [n_mats][6] = kd rgb, ka rgb of this pass, added to
     uint32_t n_mats;
     uint16_t* adj_hist;         // exact roulette: [capacity][kHistMax] kd-factor materials
     bool adj_exact;
+    uint32_t* vis;              // recorded adjoint: per path, bit b set if bounce b's light sample is visible
+    uint32_t vis_bit;           // this launch's bounce
     // octant-binned extension queues: queue q holds 8 regions of `capacity`
     // entries, region k the paths whose next ray points into octant k
     bool octant;
@@ -237,13 +238,13 @@ CRT_D void zero_grad_block(float* acc, uint32_t n_mats) {
     __syncthreads();
 }
 
+// A block's sums into the pass's, in FP64: some 60,000 blocks and bounces add to
+// each material, and their FP32 sum was off by 6-8e-6 of the gradient (now 1e-6).
 CRT_D void flush_grad_block(const WaveParams& W, const float* acc) {
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < 6u * W.n_mats; i += blockDim.x) {
         const float v = acc[i];
-        if (v == 0.f) continue;
-        const uint32_t m = i / 6u, k = i % 6u;
-        atomicAdd(k < 3u ? W.grad_kd + 3u * m + k : W.grad_ka + 3u * m + (k - 3u), v);
+        if (v != 0.f) atomicAdd(W.grad + i, (double)v);
     }
 }
 
@@ -381,6 +382,7 @@ __global__ void __launch_bounds__(kWaveBlock) wf_generate(WaveParams W) {
         Ray ray;
         begin_path(V.cam, W.R.seed, V.view_id, pixel % V.width, pixel / V.width, pixel, sample, ps, ray);
         store_state(W, i, ps, ray, pixel, sample, sg.view);
+        if (!REPLAY && W.vis) W.vis[i] = 0;
         W.queue[cur][i] = i;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -556,6 +558,15 @@ CRT_D void shade_entry(const WaveParams& W, uint32_t path, float* grad_sh, bool&
             alive = shade_hit(W.R, ps, ray, h, sr, &g) && ps.bounce < W.R.max_depth;
         }
         if (W.adj_exact) W.st_W[path].w = __uint_as_float(g.meta);
+        if (W.vis && sr.valid) {
+            // the primal trace left this light sample's visibility: what
+            // wf_shadow_adj would add, here
+            if (W.vis[path] & W.vis_bit) {
+                ps.color = ps.color + sr.contrib;
+                warp_add_grad(grad_sh, sr.light_mat, 3, xyz(wv) * sr.dcontrib);
+            }
+            sr.valid = false;
+        }
     } else if (h.face < 0) {
         shade_miss(ps);
     } else {
@@ -790,6 +801,7 @@ struct ShadowJob {
         col.y = col.y + c.y;
         col.z = col.z + c.z;
         W.st_cm[2ull * path] = col;
+        if (!ADJ && W.vis) W.vis[path] |= W.vis_bit;   // one light sample per path and bounce
         if (ADJ) {
             const float4 g = W.shd_grad[entry];
             warp_add_grad(grad, __float_as_uint(g.w), 3, xyz(g));
@@ -1558,7 +1570,13 @@ int wavefront_pass(crt_render r, const std::vector<ViewWork>& work) {
 // then the replay re-runs the path and turns each event into gradient terms
 // (WaveGrad) -- so nothing per vertex is stored.
 // ---------------------------------------------------------------------------
-static int ensure_adjoint_buffers(WaveSet& set, bool exact) {
+// Up to this many bounces the primal trace records each path's hits (16 bytes a
+// bounce) and light visibilities (a bit a bounce), and the replay reads them
+// instead of tracing the same rays again.
+constexpr uint32_t kRecordDepth = 16;
+constexpr size_t kRecordBytes = 6ull << 30;   // per wave set
+
+static int ensure_adjoint_buffers(WaveSet& set, bool exact, uint32_t max_depth) {
     WaveBuffers& B = set.buf;
     const size_t c = B.capacity;
     if (!B.adj_L.p) {
@@ -1567,6 +1585,15 @@ static int ensure_adjoint_buffers(WaveSet& set, bool exact) {
         CRT_CUDA(B.adj_shadow.alloc(c * 16));
     }
     if (exact && !B.adj_hist.p) CRT_CUDA(B.adj_hist.alloc(c * kHistMax * sizeof(uint16_t)));
+    if (max_depth <= kRecordDepth && c * 16 * max_depth <= kRecordBytes && !B.adj_hits.p && !B.adj_no_room) {
+        // without room for the record the replay traces its rays again
+        if (B.adj_hits.alloc(c * 16 * max_depth) != cudaSuccess || B.adj_vis.alloc(c * 4) != cudaSuccess) {
+            cudaGetLastError();
+            B.adj_hits.alloc(0);
+            B.adj_vis.alloc(0);
+            B.adj_no_room = true;
+        }
+    }
     return CRT_OK;
 }
 
@@ -1583,14 +1610,22 @@ static AdjointGrids adjoint_grids(crt_render r, const WaveGrids& G) {
     a.shadow_smem = G.tsmem + gsm;
     a.shadow = uses_f32_nodes(r) ? wf_shadow_adj<true> : wf_shadow_adj<false>;
     cudaFuncSetAttribute((const void*)a.shadow, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)a.shadow_smem);
-    cudaFuncSetAttribute((const void*)G.shade_adj, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)a.shade_smem);
+    cudaFuncSetAttribute((const void*)G.shade_adj, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)a.shade_smem);
+    cudaFuncSetAttribute((const void*)wf_shade<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)a.shade_smem);
     a.shd = persistent_grid((const void*)a.shadow, G.tblock, a.shadow_smem);
     return a;
 }
 
-static WaveParams adjoint_params(crt_render r, WaveSet& set, const float4* adj, float* gkd, float* gka,
-                                 uint32_t flags) {
+// The pass's gradient sums added to the caller's.
+__global__ void add_grad_kernel(const double* __restrict__ grad, uint32_t n_mats, float* __restrict__ kd,
+                                float* __restrict__ ka) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < 6u * n_mats; i += gridDim.x * blockDim.x) {
+        float* to = i % 6u < 3u ? kd + 3u * (i / 6u) + i % 6u : ka + 3u * (i / 6u) + i % 6u - 3u;
+        *to = (float)((double)*to + grad[i]);
+    }
+}
+
+static WaveParams adjoint_params(crt_render r, WaveSet& set, const float4* adj, uint32_t flags) {
     WaveParams W = wave_params(r, set);
     W.adj_exact = (flags & CRT_ADJOINT_EXACT_ROULETTE) != 0;
     W.adj_hist = set.buf.adj_hist.as<uint16_t>();
@@ -1598,25 +1633,19 @@ static WaveParams adjoint_params(crt_render r, WaveSet& set, const float4* adj, 
     W.st_L = set.buf.adj_L.as<float4>();
     W.st_W = set.buf.adj_W.as<float4>();
     W.shd_grad = set.buf.adj_shadow.as<float4>();
-    W.grad_kd = gkd;
-    W.grad_ka = gka;
+    W.grad = r->adj_grad.as<double>();
     W.n_mats = r->scene->n_mats;
     return W;
 }
 
-static int capture_adjoint_graph(crt_render r, WaveSet& set, const float4* adj, float* gkd, float* gka,
-                                 uint32_t flags) {
-    if (set.adj_graph && set.adj_key[0] == adj && set.adj_key[1] == gkd && set.adj_key[2] == gka &&
-        set.adj_flags == flags)
-        return CRT_OK;
+static int capture_adjoint_graph(crt_render r, WaveSet& set, const float4* adj, uint32_t flags) {
+    if (set.adj_graph && set.adj_key == adj && set.adj_flags == flags) return CRT_OK;
     delete static_cast<WaveGraph*>(set.adj_graph);
     WaveGraph* g = new WaveGraph();
     set.adj_graph = g;
-    set.adj_key[0] = adj;
-    set.adj_key[1] = gkd;
-    set.adj_key[2] = gka;
+    set.adj_key = adj;
     set.adj_flags = flags;
-    const WaveParams W = adjoint_params(r, set, adj, gkd, gka, flags);
+    const WaveParams W = adjoint_params(r, set, adj, flags);
     const WaveGrids G = wave_grids(r, set.buf.capacity);
     const AdjointGrids A = adjoint_grids(r, G);
     CRT_CUDA(cudaGetLastError());
@@ -1624,12 +1653,34 @@ static int capture_adjoint_graph(crt_render r, WaveSet& set, const float4* adj, 
     CRT_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
     cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-        enqueue_wave_body(W, G, r->opts.max_depth, cap);     // primal trace
-        wf_generate<true><<<G.gen, kWaveBlock, 0, cap>>>(W);  // replay
+        const bool record = set.buf.adj_hits.p != nullptr;
+        WaveParams Wb = W;   // this bounce's launches
+        auto at_bounce = [&](uint32_t b) {
+            if (!record) return;
+            Wb.hit = set.buf.adj_hits.as<float4>() + (size_t)b * set.buf.capacity;
+            Wb.vis = set.buf.adj_vis.as<uint32_t>();
+            Wb.vis_bit = 1u << b;
+        };
+        at_bounce(0);
+        wf_generate<false><<<G.gen, kWaveBlock, 0, cap>>>(Wb);   // primal trace
         for (uint32_t b = 0; b < r->opts.max_depth; ++b) {
-            G.extend<<<G.ext, G.tblock, G.tsmem, cap>>>(W);
-            G.shade_adj<<<G.sha_adj, kWaveBlock, A.shade_smem, cap>>>(W);
-            A.shadow<<<A.shd, G.tblock, A.shadow_smem, cap>>>(W);
+            at_bounce(b);
+            G.extend<<<G.ext, G.tblock, G.tsmem, cap>>>(Wb);
+            G.shade<<<G.sha, kWaveBlock, 0, cap>>>(Wb);
+            G.shadow<<<G.shd, G.tblock, G.tsmem, cap>>>(Wb);
+            wf_flip<<<1, 1, 0, cap>>>(Wb);
+        }
+        wf_generate<true><<<G.gen, kWaveBlock, 0, cap>>>(W);     // replay
+        for (uint32_t b = 0; b < r->opts.max_depth; ++b) {
+            at_bounce(b);
+            if (record) {
+                // nothing to trace: no window sort, so paths stay in order
+                wf_shade<true, false><<<G.gen, kWaveBlock, A.shade_smem, cap>>>(Wb);
+            } else {
+                G.extend<<<G.ext, G.tblock, G.tsmem, cap>>>(W);
+                G.shade_adj<<<G.sha_adj, kWaveBlock, A.shade_smem, cap>>>(W);
+                A.shadow<<<A.shd, G.tblock, A.shadow_smem, cap>>>(W);
+            }
             wf_flip<<<1, 1, 0, cap>>>(W);
         }
         e = cudaStreamEndCapture(cap, &g->graph);
@@ -1653,7 +1704,10 @@ int wavefront_adjoint(crt_render r, const std::vector<ViewWork>& work, const flo
     int st = ensure_wave_sets(r, K);
     if (st != CRT_OK) return st;
     for (WaveSet& s : r->sets)
-        if ((st = ensure_adjoint_buffers(s, exact)) != CRT_OK) return st;
+        if ((st = ensure_adjoint_buffers(s, exact, r->opts.max_depth)) != CRT_OK) return st;
+    const size_t grad_bytes = (size_t)6 * r->scene->n_mats * sizeof(double);
+    if (!r->adj_grad.p) CRT_CUDA(r->adj_grad.alloc(grad_bytes));   // a scene keeps its material count
+    CRT_CUDA(cudaMemsetAsync(r->adj_grad.p, 0, grad_bytes, r->stream));
     const uint32_t cap = r->sets[0].buf.capacity;
     const WavePlan plan = make_waves(r, work, cap);
     if (r->scene_generation != r->scene->generation) {
@@ -1669,7 +1723,7 @@ int wavefront_adjoint(crt_render r, const std::vector<ViewWork>& work, const flo
             if ((st = ensure_segments(r->sets[k], segs.size())) != CRT_OK) return st;
         }
     for (WaveSet& s : r->sets)
-        if ((st = capture_adjoint_graph(r, s, adj, gkd, gka, flags)) != CRT_OK) return st;
+        if ((st = capture_adjoint_graph(r, s, adj, flags)) != CRT_OK) return st;
     CRT_CUDA(cudaEventRecord(r->pass_start, r->stream));
     for (WaveSet& s : r->sets) CRT_CUDA(cudaStreamWaitEvent(s.stream, r->pass_start, 0));
     for (size_t c0 = 0; c0 < plan.waves.size(); c0 += chunk) {
@@ -1689,6 +1743,9 @@ int wavefront_adjoint(crt_render r, const std::vector<ViewWork>& work, const flo
         CRT_CUDA(cudaEventRecord(s.acc_done, s.stream));
         CRT_CUDA(cudaStreamWaitEvent(r->stream, s.acc_done, 0));
     }
+    add_grad_kernel<<<grid_for(6u * r->scene->n_mats, 256, 1), 256, 0, r->stream>>>(r->adj_grad.as<double>(),
+                                                                                   r->scene->n_mats, gkd, gka);
+    CRT_CUDA(cudaGetLastError());
     return CRT_OK;
 }
 
