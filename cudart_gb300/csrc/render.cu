@@ -134,13 +134,34 @@ RenderParams make_params(crt_render r, uint32_t view, uint32_t spp0, uint32_t ns
     return P;
 }
 
+static int device_error_status(uint32_t err) {
+    if (err & ERR_WATCHDOG) return set_error(CRT_ERR_WATCHDOG, "traversal exceeded its node-visit limit");
+    if (err & ERR_STACK) return set_error(CRT_ERR_WATCHDOG, "traversal stack overflow");
+    return CRT_OK;
+}
+
 int check_device_error(crt_render r) {
     uint32_t err = 0;
     CRT_CUDA(cudaMemcpyAsync(&err, r->scene->error.p, 4, cudaMemcpyDeviceToHost, r->stream));
     CRT_CUDA(cudaStreamSynchronize(r->stream));
-    if (err & ERR_WATCHDOG) return set_error(CRT_ERR_WATCHDOG, "traversal exceeded its node-visit limit");
-    if (err & ERR_STACK) return set_error(CRT_ERR_WATCHDOG, "traversal stack overflow");
+    return device_error_status(err);
+}
+
+// The handle's staging buffer, at least `bytes` long (work queued on the
+// handle's stream may still use it: freeing the old one waits for that).
+static int ensure_staging(crt_render r, size_t bytes) {
+    if (r->staging.bytes < bytes) CRT_CUDA(r->staging.alloc(bytes));
     return CRT_OK;
+}
+
+// Copies `bytes` of the staging buffer to the host behind the work queued on
+// the handle's stream, with the scene's error word, and waits once.
+static int fetch_staging(crt_render r, void* host, size_t bytes) {
+    uint32_t err = 0;
+    CRT_CUDA(cudaMemcpyAsync(&err, r->scene->error.p, 4, cudaMemcpyDeviceToHost, r->stream));
+    CRT_CUDA(cudaMemcpyAsync(host, r->staging.p, bytes, cudaMemcpyDeviceToHost, r->stream));
+    CRT_CUDA(cudaStreamSynchronize(r->stream));
+    return device_error_status(err);
 }
 
 // Copies the view table (cameras, sizes, accumulator offsets) to the device.
@@ -247,28 +268,22 @@ static int resolve_view(crt_render r, uint32_t v, uint8_t* host_rgba) {
     const ViewState& V = r->views[v];
     if (V.samples_rendered == 0) return set_error(CRT_ERR_INVALID, "no samples rendered");
     const uint32_t n = V.npix();
-    DevBuf out;
-    CRT_CUDA(out.alloc((size_t)n * 4));
+    if (int st = ensure_staging(r, (size_t)n * 4)) return st;
     resolve_kernel<<<grid_for(n, 256, 8), 256, 0, r->stream>>>(r->accum.as<float4>() + V.pix_off, n,
                                                               (float)V.samples_rendered,
-                                                              r->lut.as<uint8_t>(), out.as<uchar4>());
+                                                              r->lut.as<uint8_t>(), r->staging.as<uchar4>());
     CRT_CUDA(cudaGetLastError());
-    CRT_CUDA(cudaMemcpyAsync(host_rgba, out.p, (size_t)n * 4, cudaMemcpyDeviceToHost, r->stream));
-    CRT_CUDA(cudaStreamSynchronize(r->stream));
-    return check_device_error(r);
+    return fetch_staging(r, host_rgba, (size_t)n * 4);
 }
 
 static int accum_view(crt_render r, uint32_t v, float* host_rgb) {
     const ViewState& V = r->views[v];
     const uint32_t n = V.npix();
-    DevBuf out;
-    CRT_CUDA(out.alloc((size_t)n * 12));
+    if (int st = ensure_staging(r, (size_t)n * 12)) return st;
     unpack_accum_kernel<<<grid_for(n, 256, 8), 256, 0, r->stream>>>(r->accum.as<float4>() + V.pix_off, n,
-                                                                   out.as<float>());
+                                                                   r->staging.as<float>());
     CRT_CUDA(cudaGetLastError());
-    CRT_CUDA(cudaMemcpyAsync(host_rgb, out.p, (size_t)n * 12, cudaMemcpyDeviceToHost, r->stream));
-    CRT_CUDA(cudaStreamSynchronize(r->stream));
-    return check_device_error(r);
+    return fetch_staging(r, host_rgb, (size_t)n * 12);
 }
 
 }  // namespace crt
@@ -436,7 +451,7 @@ int crt_render_resolve_async(crt_render r, uint8_t* host_rgba) {
     const ViewState& V = r->views[0];
     if (V.samples_rendered == 0) return set_error(CRT_ERR_INVALID, "no samples rendered");
     const uint32_t n = V.npix();
-    if (r->staging.bytes < (size_t)n * 4) CRT_CUDA(r->staging.alloc((size_t)n * 4));
+    if (int st = ensure_staging(r, (size_t)n * 4)) return st;
     resolve_kernel<<<grid_for(n, 256, 8), 256, 0, r->stream>>>(r->accum.as<float4>() + V.pix_off, n,
                                                               (float)V.samples_rendered,
                                                               r->lut.as<uint8_t>(), r->staging.as<uchar4>());
