@@ -673,8 +673,8 @@ def run_gb300(args):
                     "hbm": {"achieved": round(dram_gbs, 1) if dram_gbs else None, "peak": peak,
                             "frac": round(dram_gbs / peak, 4) if dram_gbs else None,
                             "peak_kind": f"{peak_kind} HBM copy; achieved = ncu DRAM traffic / time"},
-                    "limiter": "divergent dependent gathers: see profiles/wf_extend_large_textured_1080p.md "
-                               "(issue-active, SIMT lanes, long-scoreboard stalls)",
+                    "limiter": "L1 data pipe and issue at half the lanes: see profiles/wf_extend_large_textured_1080p.md; "
+                               "lanes of a warp in one node share its loads, so frac may pass 1",
                     "algorithmic_bytes": f"nodes visited x {node_bytes} B "
                                          "+ triangles tested x 40 B per ray",
                     "staged_nodes_per_ray": round(main["staged_nodes_per_ray"], 3)}

@@ -2,7 +2,7 @@
 //
 // Replaces the reference's scene preparation (src/geometry/scene.cpp:74-165)
 // and the ParallelRenderer uploads (src/renderer/parallel_renderer.cu:37-279):
-// triangles become 48-byte intersection records in BVH leaf order plus
+// triangles become 40-byte intersection records in BVH leaf order plus
 // per-face shading records, materials a small float4 table, and the BVH an
 // 8-wide quantised tree (bvh8.cpp) instead of two 1-D textures.
 #include "crt_internal.h"
