@@ -683,45 +683,64 @@ __global__ void __launch_bounds__(kBlock) k_emit(const GWide* __restrict__ recs,
 
 uint32_t blocks(uint64_t n) { return (uint32_t)std::max<uint64_t>(1, (n + kBlock - 1) / kBlock); }
 
+// Where a build's temporaries lie in its scratch.  The first part serves in
+// turn the boxes and sort keys, the collapse's costs, and the collapse's levels.
+struct Scratch {
+    size_t sort_bytes = 0, scan_bytes = 0;
+    size_t tbox, cent, keys, vals, keys2, sort, cost, recs, cnt, off, fa, fb, scan;
+    size_t perm, nodes, ca, cb, pair, counts, dec, flags, small, bytes;
+
+    cudaError_t init(uint32_t n) {
+        cudaError_t e = cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, (const uint64_t*)nullptr, (uint64_t*)nullptr,
+                                                        (const uint32_t*)nullptr, (uint32_t*)nullptr, (int)n, 0, 63);
+        if (e == cudaSuccess)
+            e = cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, (const uint64_t*)nullptr, (uint64_t*)nullptr, (int)n + 1);
+        if (e != cudaSuccess) return e;
+        const size_t n1 = n, nn2 = 2 * n1 - 1;
+        Arena mem;
+        tbox = mem.take(n1 * sizeof(GBox)), cent = mem.take(n1 * 12), keys = mem.take(n1 * 8), vals = mem.take(n1 * 4);
+        keys2 = mem.take(n1 * 8), sort = mem.take(sort_bytes);
+        size_t end = mem.at;
+        mem.at = 0;
+        cost = mem.take(nn2 * 8 * sizeof(float));
+        end = std::max(end, mem.at);
+        mem.at = 0;
+        recs = mem.take(n1 * sizeof(GWide)), cnt = mem.take((n1 + 1) * 8), off = mem.take((n1 + 1) * 8);
+        fa = mem.take(n1 * 4), fb = mem.take(n1 * 4), scan = mem.take(scan_bytes);
+        mem.at = std::max(end, mem.at);
+        perm = mem.take(n1 * 4), nodes = mem.take(nn2 * sizeof(GNode)), ca = mem.take(n1 * 4), cb = mem.take(n1 * 4);
+        pair = mem.take(n1 * 4), counts = mem.take((n1 / kBlock + 1) * 8), dec = mem.take(nn2 * sizeof(GDec));
+        flags = mem.take(n1 * 4), small = mem.take(64);
+        bytes = mem.at;
+        return cudaSuccess;
+    }
+};
+
 }  // namespace
+
+size_t bvh_gpu_scratch(uint32_t n) {
+    Scratch L;
+    if (n == 0 || n >= (1u << 30)) return 0;   // build_bvh_gpu refuses these
+    return L.init(n) == cudaSuccess ? L.bytes : 0;
+}
 
 // Builds the BVH of n triangles (device arrays v1/e1/e2, [n][3]) into nodes,
 // fnodes and tris (device, allocated here; tris holds n DevTriA, then n
-// DevTriB); fills max_depth and the node count.  Returns CRT_OK or an error with its message set.
+// DevTriB); fills max_depth and the node count.  scratch: bvh_gpu_scratch(n)
+// bytes, 256-byte aligned.  Returns CRT_OK or an error with its message set.
 int build_bvh_gpu(const float* d_v1, const float* d_e1, const float* d_e2, uint32_t n, uint32_t max_levels,
-                  int max_children, DevBuf& nodes_out, DevBuf& fnodes_out, DevBuf& tris_out, uint32_t* num_nodes,
+                  int max_children, void* scratch, DevBuf& nodes_out, DevBuf& fnodes_out, DevBuf& tris_out, uint32_t* num_nodes,
                   uint32_t* max_depth, bool* fnodes_ok, cudaStream_t s) {
     if (n == 0) return set_error(CRT_ERR_INVALID, "scene has no triangles");
     if (n >= (1u << 30)) return set_error(CRT_ERR_LIMIT, "GPU BVH build: at most 2^30 triangles");
     const int ni = (int)n;
     const size_t n1 = n, nn2 = 2 * n1 - 1;
-    size_t sort_bytes = 0, scan_bytes = 0;
-    CRT_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, (const uint64_t*)nullptr, (uint64_t*)nullptr,
-                                             (const uint32_t*)nullptr, (uint32_t*)nullptr, ni, 0, 63, s));
-    CRT_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, (const uint64_t*)nullptr, (uint64_t*)nullptr, ni + 1, s));
-    // One allocation for every temporary.  The first part serves in turn the
-    // boxes and sort keys, the collapse's costs, and the collapse's levels.
-    Arena mem;
-    const size_t phase0 = mem.at;
-    const size_t o_tbox = mem.take(n1 * sizeof(GBox)), o_cent = mem.take(n1 * 12), o_keys = mem.take(n1 * 8),
-                 o_vals = mem.take(n1 * 4), o_keys2 = mem.take(n1 * 8), o_sort = mem.take(sort_bytes);
-    size_t end = mem.at;
-    mem.at = phase0;
-    const size_t o_cost = mem.take(nn2 * 8 * sizeof(float));
-    end = std::max(end, mem.at);
-    mem.at = phase0;
-    const size_t o_recs = mem.take(n1 * sizeof(GWide)), o_cnt = mem.take((n1 + 1) * 8), o_off = mem.take((n1 + 1) * 8),
-                 o_fa = mem.take(n1 * 4), o_fb = mem.take(n1 * 4), o_scan = mem.take(scan_bytes);
-    mem.at = std::max(end, mem.at);
-    const size_t o_perm = mem.take(n1 * 4), o_nodes = mem.take(nn2 * sizeof(GNode)), o_ca = mem.take(n1 * 4),
-                 o_cb = mem.take(n1 * 4), o_pair = mem.take(n1 * 4), o_counts = mem.take((n1 / kBlock + 1) * 8),
-                 o_dec = mem.take(nn2 * sizeof(GDec)), o_flags = mem.take(n1 * 4), o_small = mem.take(64);
-    DevBuf arena;
-    CRT_CUDA(arena.alloc(mem.at));
-    char* base = arena.as<char>();
-    uint32_t* err = reinterpret_cast<uint32_t*>(base + o_small);       // word 0: error bits, 1: largest magnitude
+    Scratch L;
+    CRT_CUDA(L.init(n));
+    char* base = static_cast<char*>(scratch);
+    uint32_t* err = reinterpret_cast<uint32_t*>(base + L.small);       // word 0: error bits, 1: largest magnitude
     uint32_t* cbounds = err + 2;                                       // words 2-7: centroid bounds
-    PlocState* ploc = reinterpret_cast<PlocState*>(base + o_small + 32);
+    PlocState* ploc = reinterpret_cast<PlocState*>(base + L.small + 32);
     const uint32_t init[8] = {0u, 0u, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u};
     CRT_CUDA(cudaMemcpyAsync(err, init, sizeof(init), cudaMemcpyHostToDevice, s));
     k_max_abs<<<blocks(3ull * n) < 1024 ? blocks(3ull * n) : 1024, kBlock, 0, s>>>(d_v1, d_e1, d_e2, 3 * n, err + 1);
@@ -732,16 +751,16 @@ int build_bvh_gpu(const float* d_v1, const float* d_e1, const float* d_e2, uint3
     std::memcpy(&maxabs, &mb, 4);
     const float margin = (float)std::ldexp(std::max(1.0, (double)maxabs), -15);
 
-    GBox* tbox = reinterpret_cast<GBox*>(base + o_tbox);
-    float* cent = reinterpret_cast<float*>(base + o_cent);
-    uint64_t* keys = reinterpret_cast<uint64_t*>(base + o_keys);
-    uint64_t* keys2 = reinterpret_cast<uint64_t*>(base + o_keys2);
-    uint32_t* vals = reinterpret_cast<uint32_t*>(base + o_vals);
-    uint32_t* perm = reinterpret_cast<uint32_t*>(base + o_perm);
+    GBox* tbox = reinterpret_cast<GBox*>(base + L.tbox);
+    float* cent = reinterpret_cast<float*>(base + L.cent);
+    uint64_t* keys = reinterpret_cast<uint64_t*>(base + L.keys);
+    uint64_t* keys2 = reinterpret_cast<uint64_t*>(base + L.keys2);
+    uint32_t* vals = reinterpret_cast<uint32_t*>(base + L.vals);
+    uint32_t* perm = reinterpret_cast<uint32_t*>(base + L.perm);
     k_tri_boxes<<<std::min<uint32_t>(blocks(n), 1216), kBlock, 0, s>>>(d_v1, d_e1, d_e2, n, margin, tbox, cent, cbounds);
     k_morton<<<std::min<uint32_t>(blocks(n), 4096), kBlock, 0, s>>>(cent, n, cbounds, keys, vals);
-    CRT_CUDA(cub::DeviceRadixSort::SortPairs(base + o_sort, sort_bytes, keys, keys2, vals, perm, ni, 0, 63, s));
-    GNode* gn = reinterpret_cast<GNode*>(base + o_nodes);
+    CRT_CUDA(cub::DeviceRadixSort::SortPairs(base + L.sort, L.sort_bytes, keys, keys2, vals, perm, ni, 0, 63, s));
+    GNode* gn = reinterpret_cast<GNode*>(base + L.nodes);
     k_leaves<<<blocks(n), kBlock, 0, s>>>(tbox, perm, ni, gn);
     int32_t root = ni - 1;   // a lone triangle is its own root
     if (n > 1) {
@@ -751,10 +770,10 @@ int build_bvh_gpu(const float* d_v1, const float* d_e1, const float* d_e2, uint3
         // library scan, the merge and a host read each iteration: 2.6 ms of 2.17M
         // triangles' build; three kernels and a read every fourth: 1.1.)
         constexpr int kPerSync = 4;
-        int32_t* cur = reinterpret_cast<int32_t*>(base + o_ca);
-        int32_t* nxt = reinterpret_cast<int32_t*>(base + o_cb);
-        int32_t* pair = reinterpret_cast<int32_t*>(base + o_pair);
-        uint64_t* counts = reinterpret_cast<uint64_t*>(base + o_counts);
+        int32_t* cur = reinterpret_cast<int32_t*>(base + L.ca);
+        int32_t* nxt = reinterpret_cast<int32_t*>(base + L.cb);
+        int32_t* pair = reinterpret_cast<int32_t*>(base + L.pair);
+        uint64_t* counts = reinterpret_cast<uint64_t*>(base + L.counts);
         k_ploc_init<<<blocks(n), kBlock, 0, s>>>(cur, ni, ploc);
         PlocState at{ni, ni - 2};
         for (uint32_t iter = 0; at.m > 1;) {
@@ -778,9 +797,9 @@ int build_bvh_gpu(const float* d_v1, const float* d_e1, const float* d_e2, uint3
         if (root != 0 || at.next_id != -1) return set_error(CRT_ERR_CUDA, "GPU BVH build: clustering left no single root");
     }
     // the collapse's costs and decisions, bottom-up
-    float* cost = reinterpret_cast<float*>(base + o_cost);
-    GDec* dec = reinterpret_cast<GDec*>(base + o_dec);
-    uint32_t* flags = reinterpret_cast<uint32_t*>(base + o_flags);
+    float* cost = reinterpret_cast<float*>(base + L.cost);
+    GDec* dec = reinterpret_cast<GDec*>(base + L.dec);
+    uint32_t* flags = reinterpret_cast<uint32_t*>(base + L.flags);
     CRT_CUDA(cudaMemsetAsync(flags, 0, n1 * 4, s));
     (max_children == 4 ? k_dp_up<4> : k_dp_up<8>)<<<blocks(n), kBlock, 0, s>>>(ni, gn, cost, dec, flags, err);
     CRT_CUDA(cudaGetLastError());
@@ -793,11 +812,11 @@ int build_bvh_gpu(const float* d_v1, const float* d_e1, const float* d_e2, uint3
 
     // ---- collapse level by level, then encode all nodes at once ------------
     const uint32_t cap_nodes = n;   // a wide node holds >= 1 triangle of its own subtree
-    GWide* recs = reinterpret_cast<GWide*>(base + o_recs);
-    uint64_t* cnt = reinterpret_cast<uint64_t*>(base + o_cnt);
-    uint64_t* off = reinterpret_cast<uint64_t*>(base + o_off);
-    int32_t* cur = reinterpret_cast<int32_t*>(base + o_fa);
-    int32_t* nxt = reinterpret_cast<int32_t*>(base + o_fb);
+    GWide* recs = reinterpret_cast<GWide*>(base + L.recs);
+    uint64_t* cnt = reinterpret_cast<uint64_t*>(base + L.cnt);
+    uint64_t* off = reinterpret_cast<uint64_t*>(base + L.off);
+    int32_t* cur = reinterpret_cast<int32_t*>(base + L.fa);
+    int32_t* nxt = reinterpret_cast<int32_t*>(base + L.fb);
     CRT_CUDA(cudaMemcpyAsync(cur, &root, 4, cudaMemcpyHostToDevice, s));
     uint32_t F = 1, level_base = 0, tri_base = 0, depth = 0;
     while (F > 0) {
@@ -805,7 +824,7 @@ int build_bvh_gpu(const float* d_v1, const float* d_e1, const float* d_e2, uint3
         k_choose<<<blocks(8ull * F), kBlock, 0, s>>>(cur, F, gn, dec, max_children, recs + level_base, cnt, ni, err);
         // exclusive sums over F + 1 entries: the last is the level's totals
         CRT_CUDA(cudaMemsetAsync(cnt + F, 0, 8, s));
-        CRT_CUDA(cub::DeviceScan::ExclusiveSum(base + o_scan, scan_bytes, cnt, off, (int)F + 1, s));
+        CRT_CUDA(cub::DeviceScan::ExclusiveSum(base + L.scan, L.scan_bytes, cnt, off, (int)F + 1, s));
         const uint32_t next_base = level_base + F;
         k_front<<<blocks(8ull * F), kBlock, 0, s>>>(recs + level_base, F, next_base, tri_base, off, dec, nxt,
                                                     cap_nodes, err);

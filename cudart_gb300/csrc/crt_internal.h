@@ -100,8 +100,9 @@ struct WaveSet {
 };
 
 namespace crt {
+size_t bvh_gpu_scratch(uint32_t n);   // bytes of scratch build_bvh_gpu needs
 int build_bvh_gpu(const float* d_v1, const float* d_e1, const float* d_e2, uint32_t n, uint32_t max_levels,
-                  int max_children, DevBuf& nodes_out, DevBuf& fnodes_out, DevBuf& tris_out, uint32_t* num_nodes,
+                  int max_children, void* scratch, DevBuf& nodes_out, DevBuf& fnodes_out, DevBuf& tris_out, uint32_t* num_nodes,
                   uint32_t* max_depth, bool* fnodes_ok, cudaStream_t s);
 void destroy_wave_sets(struct ::crt_render_s* r);
 void drop_wave_graphs(struct ::crt_render_s* r);

@@ -201,12 +201,13 @@ static int ensure_host_bvh(crt_scene s) {
 }
 
 // Builds the BVH of device arrays v1/e1/e2 ([n][3]) on the GPU and installs it.
+// scratch: bvh_gpu_scratch(n) bytes.
 static int build_on_device(crt_scene s, const float* dv1, const float* de1, const float* de2, uint32_t n,
-                           uint32_t width) {
+                           uint32_t width, void* scratch) {
     DevBuf nodes, fnodes, tris;
     uint32_t nn = 0, depth = 0;
     bool fok = false;
-    if (int st = build_bvh_gpu(dv1, de1, de2, n, (uint32_t)kMaxLevels, (int)width, nodes, fnodes, tris, &nn, &depth,
+    if (int st = build_bvh_gpu(dv1, de1, de2, n, (uint32_t)kMaxLevels, (int)width, scratch, nodes, fnodes, tris, &nn, &depth,
                                &fok, nullptr))
         return st;
     if (s->default_f32 && !fok)
@@ -237,7 +238,9 @@ static int build_and_install(crt_scene s, const std::vector<float>& v1, const st
         DevBuf dv1, de1, de2;
         int st = CRT_OK;
         if ((st = upload(dv1, v1)) || (st = upload(de1, e1)) || (st = upload(de2, e2))) return st;
-        return build_on_device(s, dv1.as<float>(), de1.as<float>(), de2.as<float>(), n, width);
+        DevBuf scratch;
+        CRT_CUDA(scratch.alloc(bvh_gpu_scratch(n)));
+        return build_on_device(s, dv1.as<float>(), de1.as<float>(), de2.as<float>(), n, width, scratch.p);
     }
     Bvh8 bvh;
     const char* msg = nullptr;
@@ -257,13 +260,25 @@ inline float bits(int32_t i) { float f; std::memcpy(&f, &i, 4); return f; }
 // Scene::loadTriangles (scene.cpp:111-130): v1, e1 = v2 - v1, e2 = v3 - v1
 // (or the edges as given), area = |e1 x e2| / 2; shading records (three
 // normals, area, material id) and uvs.
-// A face with a non-finite coordinate sets *bad (the builds bin by centroid
-// and must not see NaN or infinity).
+// found[0]: the lowest face with a non-finite coordinate (the builds bin by
+// centroid and must not see NaN or infinity); found[1]: the lowest with a
+// material id out of range; found[2 + i / 32], bit i % 32, with emits (a byte per
+// material): face i emits.  HBM-bound (2.17M faces: 92 us).  The id check and the
+// emitters were two passes of the host over the ids, 1.25 of a 7.0 ms creation;
+// here they are two instructions per face and a copy of a bit per face.
 __global__ void k_pack_faces(const float* __restrict__ pos, const float* __restrict__ nor,
                              const float* __restrict__ uv, const uint32_t* __restrict__ mid, uint32_t n, bool edges,
                              float* __restrict__ v1, float* __restrict__ e1, float* __restrict__ e2,
-                             float4* __restrict__ shade, float4* __restrict__ uvs, uint32_t* bad) {
+                             float4* __restrict__ shade, float4* __restrict__ uvs, uint32_t n_mats,
+                             const uint8_t* __restrict__ emits, uint32_t* found) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t id = mid[i];
+        if (emits) {   // a warp's faces are 32 in a row from a multiple of 32, or what is left of them
+            const uint32_t in_row = min(n - (i & ~31u), 32u);
+            const uint32_t word = __ballot_sync(0xFFFFFFFFu >> (32u - in_row), id < n_mats && emits[id]);
+            if ((i & 31u) == 0) found[2 + (i >> 5)] = word;
+        }
+        if (id >= n_mats) atomicMin(found + 1, i);
         const float* p = pos + 9ull * i;
         float a[3], b[3];
         bool finite = true;
@@ -276,13 +291,13 @@ __global__ void k_pack_faces(const float* __restrict__ pos, const float* __restr
             e1[3ull * i + k] = a[k];
             e2[3ull * i + k] = b[k];
         }
-        if (!finite) atomicMin(bad, i);
+        if (!finite) atomicMin(found, i);
         const float cx = a[1] * b[2] - a[2] * b[1], cy = a[2] * b[0] - a[0] * b[2], cz = a[0] * b[1] - a[1] * b[0];
         const float area = sqrtf(cx * cx + cy * cy + cz * cz) / 2.0f;
         const float* nn = nor + 9ull * i;
         shade[3ull * i + 0] = make_float4(nn[0], nn[1], nn[2], nn[3]);
         shade[3ull * i + 1] = make_float4(nn[4], nn[5], nn[6], nn[7]);
-        shade[3ull * i + 2] = make_float4(nn[8], area, __uint_as_float(mid[i]), 0.f);
+        shade[3ull * i + 2] = make_float4(nn[8], area, __uint_as_float(id), 0.f);
         if (uv) {
             const float* t = uv + 6ull * i;
             uvs[2ull * i + 0] = make_float4(t[0], t[1], t[2], t[3]);
@@ -318,17 +333,6 @@ static float face_area(const crt_scene_desc* d, uint32_t f, float e1[3], float e
     const float cx = e1[1] * e2[2] - e1[2] * e2[1], cy = e1[2] * e2[0] - e1[0] * e2[2],
                 cz = e1[0] * e2[1] - e1[1] * e2[0];
     return sqrtf(cx * cx + cy * cy + cz * cz) / 2.0f;
-}
-
-template <typename T>
-static int upload_raw(DevBuf& b, const T* p, size_t count) {
-    cudaError_t e = b.alloc(count ? count * sizeof(T) : 16);
-    if (e != cudaSuccess) return cuda_error(e, "cudaMalloc");
-    if (count) {
-        e = cudaMemcpy(b.p, p, count * sizeof(T), cudaMemcpyHostToDevice);
-        if (e != cudaSuccess) return cuda_error(e, "cudaMemcpy");
-    }
-    return CRT_OK;
 }
 
 // Materials (createMaterialsData, parallel_renderer.cu:252-279) with the
@@ -395,67 +399,56 @@ int crt_scene_create(const crt_scene_desc* d, crt_scene* out) {
     if (d->num_materials == 0 || !d->materials)
         return set_error(CRT_ERR_INVALID, "scene has no materials");
     if (n >= (1u << 31)) return set_error(CRT_ERR_LIMIT, "more than 2^31 triangles");
-    uint32_t top_id = 0;   // a plain maximum vectorises; the offender is looked up only if there is one
-    for (uint32_t i = 0; i < n; ++i) top_id = std::max(top_id, d->material_ids[i]);
-    if (top_id >= d->num_materials)
+    // Material ids and emitters are looked over on the device (k_pack_faces).
+    // Where the host refuses something else first, it looks them over itself: the
+    // first fault in this order is the one reported, with a device or without.
+    auto bad_id = [](uint32_t i) {
+        return set_error(CRT_ERR_INVALID, "material id out of range at face " + std::to_string(i));
+    };
+    auto no_emitter = [] {
+        return set_error(CRT_ERR_INVALID, "scene has no emissive triangles (light sampling needs one)");
+    };
+    auto ids_status = [&]() -> int {
         for (uint32_t i = 0; i < n; ++i)
-            if (d->material_ids[i] >= d->num_materials)
-                return set_error(CRT_ERR_INVALID, "material id out of range at face " + std::to_string(i));
+            if (d->material_ids[i] >= d->num_materials) return bad_id(i);
+        return CRT_OK;
+    };
+    auto lights_status = [&]() -> int {
+        if (int st = ids_status()) return st;
+        if (d->num_lights) return CRT_OK;
+        for (uint32_t i = 0; i < n; ++i)
+            if (d->materials[d->material_ids[i]].bsdf == CRT_BSDF_EMISSIVE) return CRT_OK;
+        return no_emitter();
+    };
+    auto refuse = [&](int code, const std::string& msg) {
+        if (int st = ids_status()) return st;
+        return set_error(code, msg);
+    };
     for (uint32_t m = 0; m < d->num_materials; ++m) {
         int t = d->materials[m].texture;
         if (t != CRT_NO_TEXTURE && (t < 0 || (uint32_t)t >= d->num_textures))
-            return set_error(CRT_ERR_INVALID, "texture index out of range in material " + std::to_string(m));
+            return refuse(CRT_ERR_INVALID, "texture index out of range in material " + std::to_string(m));
         if (d->materials[m].bsdf < 0 || d->materials[m].bsdf > CRT_BSDF_EMISSIVE)
-            return set_error(CRT_ERR_INVALID, "unknown bsdf in material " + std::to_string(m));
+            return refuse(CRT_ERR_INVALID, "unknown bsdf in material " + std::to_string(m));
     }
     if (d->num_textures && (!d->texture_dims || (!d->texels && !d->texels_rgba8)))
-        return set_error(CRT_ERR_INVALID, "textures need dims and texels");
-    if (d->node_format > CRT_NODES_F32) return set_error(CRT_ERR_INVALID, "unknown node format");
+        return refuse(CRT_ERR_INVALID, "textures need dims and texels");
+    if (d->node_format > CRT_NODES_F32) return refuse(CRT_ERR_INVALID, "unknown node format");
     if (d->flags & ~(uint32_t)(CRT_SCENE_EDGES | CRT_SCENE_KA_SCALED))
-        return set_error(CRT_ERR_INVALID, "unknown scene flag");
-    if (d->builder > CRT_BVH_GPU) return set_error(CRT_ERR_INVALID, "unknown BVH builder");
+        return refuse(CRT_ERR_INVALID, "unknown scene flag");
+    if (d->builder > CRT_BVH_GPU) return refuse(CRT_ERR_INVALID, "unknown BVH builder");
     if (d->bvh_width != 0 && d->bvh_width != 4 && d->bvh_width != 8)
-        return set_error(CRT_ERR_INVALID, "bvh_width must be 4 or 8");
+        return refuse(CRT_ERR_INVALID, "bvh_width must be 4 or 8");
 
     auto t0 = std::chrono::steady_clock::now();
     crt_scene s = new crt_scene_s();
 
-    // Light list (scene.cpp:148-160) and total light area (scene.cpp:167-173),
-    // with each light's geometry as Scene::loadTriangles computes it.
     if (d->num_lights) {
-        if (!d->light_indices) { delete s; return set_error(CRT_ERR_INVALID, "light_indices is null"); }
+        if (!d->light_indices) { delete s; return refuse(CRT_ERR_INVALID, "light_indices is null"); }
         for (uint32_t i = 0; i < d->num_lights; ++i) {
-            if (d->light_indices[i] >= n) { delete s; return set_error(CRT_ERR_INVALID, "light index out of range"); }
+            if (d->light_indices[i] >= n) { delete s; return refuse(CRT_ERR_INVALID, "light index out of range"); }
             s->lights.push_back(d->light_indices[i]);
         }
-    } else {
-        // emitters are few: a byte per material, tested by the block
-        std::vector<uint8_t> emits(d->num_materials);
-        for (uint32_t m = 0; m < d->num_materials; ++m) emits[m] = d->materials[m].bsdf == CRT_BSDF_EMISSIVE;
-        for (uint32_t i0 = 0; i0 < n; i0 += 64) {
-            const uint32_t i1 = std::min(n, i0 + 64);
-            uint32_t any = 0;
-            for (uint32_t i = i0; i < i1; ++i) any |= emits[d->material_ids[i]];
-            if (!any) continue;
-            for (uint32_t i = i0; i < i1; ++i)
-                if (emits[d->material_ids[i]]) s->lights.push_back(i);
-        }
-    }
-    if (s->lights.empty()) {
-        delete s;
-        return set_error(CRT_ERR_INVALID, "scene has no emissive triangles (light sampling needs one)");
-    }
-    std::vector<float4> lgeo(3 * s->lights.size());
-    float lights_area = 0;
-    for (size_t i = 0; i < s->lights.size(); ++i) {
-        const uint32_t f = s->lights[i];
-        float e1[3], e2[3];
-        const float area = face_area(d, f, e1, e2);
-        const float* p = d->positions + 9ull * f;
-        lgeo[3 * i + 0] = f4(p[0], p[1], p[2], bits(f));
-        lgeo[3 * i + 1] = f4(e1[0], e1[1], e1[2], area);
-        lgeo[3 * i + 2] = f4(e2[0], e2[1], e2[2], bits(d->material_ids[f]));
-        lights_area += area;
     }
     // Textures flattened in order, then as many zero texels as the last
     // texture is wide (texture_store.cpp:68-70).
@@ -464,16 +457,28 @@ int crt_scene_create(const crt_scene_desc* d, crt_scene* out) {
     uint64_t total = 0;
     for (uint32_t t = 0; t < d->num_textures; ++t) {
         uint32_t w = d->texture_dims[2 * t], h = d->texture_dims[2 * t + 1];
-        if (w == 0 || h == 0) { delete s; return set_error(CRT_ERR_INVALID, "empty texture"); }
+        if (w == 0 || h == 0) {
+            delete s;
+            if (int st = lights_status()) return st;
+            return set_error(CRT_ERR_INVALID, "empty texture");
+        }
         dims.push_back(make_uint2(w, h));
         offs.push_back((uint32_t)total);
         total += (uint64_t)w * h;
-        if (total >= (1ull << 31)) { delete s; return set_error(CRT_ERR_LIMIT, "texture data too large"); }
+        if (total >= (1ull << 31)) {
+            delete s;
+            if (int st = lights_status()) return st;
+            return set_error(CRT_ERR_LIMIT, "texture data too large");
+        }
     }
     const uint64_t pad = d->num_textures ? dims.back().x : 0;
-    // Host-side validation is complete; from here on a device is needed.
+    // From here on a device is needed.
     cudaError_t dev_err = cudaGetDevice(&s->device);
-    if (dev_err != cudaSuccess) { delete s; return cuda_error(dev_err, "cudaGetDevice"); }
+    if (dev_err != cudaSuccess) {
+        delete s;
+        if (int st = lights_status()) return st;
+        return cuda_error(dev_err, "cudaGetDevice");
+    }
 
     const uint32_t width = d->bvh_width ? d->bvh_width : 8u;
     s->builder = d->builder;
@@ -488,42 +493,66 @@ int crt_scene_create(const crt_scene_desc* d, crt_scene* out) {
     // shading and uv records there.
     int st = CRT_OK;
     {
-        // (one allocation for what the caller's arrays and the edges need here)
+        // One allocation for what is needed here only: the edges and k_pack_faces'
+        // findings, then a region that holds in turn the caller's arrays, the BVH
+        // build's scratch and the raw texels (four allocations of their own, freed
+        // one by one, took 0.6 of a 7.0 ms creation of 2.17M triangles).
+        const size_t n_found = 2 + (d->num_lights ? 0 : (n + 31ull) / 32);
         Arena mem;
+        const size_t o_v1 = mem.take(12ull * n), o_e1 = mem.take(12ull * n), o_e2 = mem.take(12ull * n),
+                     o_found = mem.take(4 * n_found);
+        const size_t o_region = mem.at;
         const size_t o_pos = mem.take(36ull * n), o_nor = mem.take(36ull * n), o_uv = mem.take(d->uvs ? 24ull * n : 0),
-                     o_mid = mem.take(4ull * n), o_v1 = mem.take(12ull * n), o_e1 = mem.take(12ull * n),
-                     o_e2 = mem.take(12ull * n), o_bad = mem.take(4);
+                     o_mid = mem.take(4ull * n), o_emits = mem.take(d->num_materials);
+        size_t end = mem.at;
+        if (s->builder == CRT_BVH_GPU) end = std::max(end, o_region + bvh_gpu_scratch(n));
+        mem.at = o_region;
+        const size_t o_table = mem.take(256 * 4), o_texels = mem.take((d->texels_rgba8 ? 4ull : 12ull) * total);
+        end = std::max(end, mem.at);
         DevBuf temp;
-        cudaError_t e = temp.alloc(mem.at);
+        cudaError_t e = temp.alloc(end);
         if (e == cudaSuccess) e = s->shade.alloc(48ull * n);
         if (e == cudaSuccess) e = s->uvs.alloc(32ull * n);
-        if (e != cudaSuccess) { delete s; return cuda_error(e, "cudaMalloc"); }
+        if (e != cudaSuccess) {
+            delete s;
+            if (int bad = lights_status()) return bad;
+            return cuda_error(e, "cudaMalloc");
+        }
         char* base = temp.as<char>();
         float* v1 = reinterpret_cast<float*>(base + o_v1);
         float* e1 = reinterpret_cast<float*>(base + o_e1);
         float* e2 = reinterpret_cast<float*>(base + o_e2);
-        uint32_t* bad = reinterpret_cast<uint32_t*>(base + o_bad);
+        uint32_t* d_found = reinterpret_cast<uint32_t*>(base + o_found);
+        std::vector<uint8_t> emits(d->num_lights ? 0 : d->num_materials);
+        for (size_t m = 0; m < emits.size(); ++m) emits[m] = d->materials[m].bsdf == CRT_BSDF_EMISSIVE;
         e = cudaMemcpy(base + o_pos, d->positions, 36ull * n, cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = cudaMemcpy(base + o_nor, d->normals, 36ull * n, cudaMemcpyHostToDevice);
         if (e == cudaSuccess && d->uvs) e = cudaMemcpy(base + o_uv, d->uvs, 24ull * n, cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = cudaMemcpy(base + o_mid, d->material_ids, 4ull * n, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemset(bad, 0xFF, 4);   // lowest bad face, or UINT32_MAX
+        if (e == cudaSuccess && !emits.empty()) e = cudaMemcpy(base + o_emits, emits.data(), emits.size(), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMemset(d_found, 0xFF, 8);   // lowest faces, or UINT32_MAX
         if (e != cudaSuccess) { delete s; return cuda_error(e, "cudaMemcpy"); }
         const uint32_t grid = (uint32_t)std::min<uint64_t>((n + 255ull) / 256, 4096);
         k_pack_faces<<<grid, 256>>>(reinterpret_cast<float*>(base + o_pos), reinterpret_cast<float*>(base + o_nor),
                                     d->uvs ? reinterpret_cast<float*>(base + o_uv) : nullptr,
                                     reinterpret_cast<uint32_t*>(base + o_mid), n, (d->flags & CRT_SCENE_EDGES) != 0, v1, e1,
-                                    e2, s->shade.as<float4>(), s->uvs.as<float4>(), bad);
+                                    e2, s->shade.as<float4>(), s->uvs.as<float4>(), d->num_materials,
+                                    emits.empty() ? nullptr : reinterpret_cast<uint8_t*>(base + o_emits), d_found);
         e = cudaGetLastError();
-        uint32_t bad_face = UINT32_MAX;
-        if (e == cudaSuccess) e = cudaMemcpy(&bad_face, bad, 4, cudaMemcpyDeviceToHost);
+        std::vector<uint32_t> found(n_found);
+        if (e == cudaSuccess) e = cudaMemcpy(found.data(), d_found, 4 * n_found, cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) { delete s; return cuda_error(e, "k_pack_faces"); }
-        if (bad_face != UINT32_MAX) {
+        if (found[1] != UINT32_MAX) { delete s; return bad_id(found[1]); }
+        for (size_t k = 2; k < n_found; ++k)   // emitters, in face order
+            for (uint32_t w = found[k]; w; w &= w - 1)
+                s->lights.push_back((uint32_t)(32 * (k - 2)) + (uint32_t)__builtin_ctz(w));
+        if (s->lights.empty()) { delete s; return no_emitter(); }
+        if (found[0] != UINT32_MAX) {
             delete s;
-            return set_error(CRT_ERR_INVALID, "non-finite vertex coordinate in face " + std::to_string(bad_face));
+            return set_error(CRT_ERR_INVALID, "non-finite vertex coordinate in face " + std::to_string(found[0]));
         }
         if (s->builder == CRT_BVH_GPU) {
-            st = build_on_device(s, v1, e1, e2, n, width);
+            st = build_on_device(s, v1, e1, e2, n, width, base + o_region);
         } else {
             std::vector<float> hv1(3ull * n), he1(3ull * n), he2(3ull * n);
             e = cudaMemcpy(hv1.data(), v1, 12ull * n, cudaMemcpyDeviceToHost);
@@ -533,31 +562,42 @@ int crt_scene_create(const crt_scene_desc* d, crt_scene* out) {
             st = build_and_install(s, hv1, he1, he2, n, width);
         }
         if (st != CRT_OK) { delete s; return st; }
-    }
-    {   // texels: floats or RGBA8 bytes up, float4 records formed on the device
-        DevBuf raw, table;
-        cudaError_t e = s->texels.alloc(16ull * (total + pad) + (total + pad == 0 ? 16 : 0));
+        // texels: floats or RGBA8 bytes up, float4 records formed on the device
+        e = s->texels.alloc(16ull * (total + pad) + (total + pad == 0 ? 16 : 0));
         if (e == cudaSuccess && pad) e = cudaMemset(s->texels.as<float4>() + total, 0, 16ull * pad);
         if (e != cudaSuccess) { delete s; return cuda_error(e, "texels"); }
         if (total) {
+            char* raw = base + o_texels;
+            float* table = reinterpret_cast<float*>(base + o_table);
             if (d->texels_rgba8) {
-                if ((st = upload_raw(raw, d->texels_rgba8, 4ull * total)) ||
-                    (st = upload_raw(table, stb_texel_table(), 256))) {
-                    delete s;
-                    return st;
-                }
-            } else if ((st = upload_raw(raw, d->texels, 3ull * total))) {
-                delete s;
-                return st;
+                e = cudaMemcpy(raw, d->texels_rgba8, 4ull * total, cudaMemcpyHostToDevice);
+                if (e == cudaSuccess) e = cudaMemcpy(table, stb_texel_table(), 256 * 4, cudaMemcpyHostToDevice);
+            } else {
+                e = cudaMemcpy(raw, d->texels, 12ull * total, cudaMemcpyHostToDevice);
             }
-            const uint32_t grid = (uint32_t)std::min<uint64_t>((total + 255) / 256, 4096);
-            k_pack_texels<<<grid, 256>>>(d->texels_rgba8 ? nullptr : raw.as<float>(),
-                                         d->texels_rgba8 ? raw.as<uchar4>() : nullptr, table.as<float>(), total,
-                                         s->texels.as<float4>());
+            if (e != cudaSuccess) { delete s; return cuda_error(e, "cudaMemcpy"); }
+            const uint32_t tgrid = (uint32_t)std::min<uint64_t>((total + 255) / 256, 4096);
+            k_pack_texels<<<tgrid, 256>>>(d->texels_rgba8 ? nullptr : reinterpret_cast<float*>(raw),
+                                          d->texels_rgba8 ? reinterpret_cast<uchar4*>(raw) : nullptr, table, total,
+                                          s->texels.as<float4>());
             e = cudaGetLastError();
             if (e == cudaSuccess) e = cudaDeviceSynchronize();
             if (e != cudaSuccess) { delete s; return cuda_error(e, "k_pack_texels"); }
         }
+    }
+    // Light geometry as Scene::loadTriangles computes it, and the total light
+    // area (scene.cpp:148-173).
+    std::vector<float4> lgeo(3 * s->lights.size());
+    float lights_area = 0;
+    for (size_t i = 0; i < s->lights.size(); ++i) {
+        const uint32_t f = s->lights[i];
+        float e1[3], e2[3];
+        const float area = face_area(d, f, e1, e2);
+        const float* p = d->positions + 9ull * f;
+        lgeo[3 * i + 0] = f4(p[0], p[1], p[2], bits(f));
+        lgeo[3 * i + 1] = f4(e1[0], e1[1], e1[2], area);
+        lgeo[3 * i + 2] = f4(e2[0], e2[1], e2[2], bits(d->material_ids[f]));
+        lights_area += area;
     }
     const std::vector<float4> mats =
         pack_materials(d->materials, d->num_materials, lights_area, (d->flags & CRT_SCENE_KA_SCALED) != 0);
