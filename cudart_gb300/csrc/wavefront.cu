@@ -1411,65 +1411,80 @@ static int build_pass_graph(crt_render r, size_t n_waves, uint32_t K) {
 // launches instead of four per bounce, and no bounce waits for the slowest ray
 // of all paths.  What bounds it is the latency of one warp's serial visits, so
 // while the chip has warps to spare a warp holds fewer paths and diverges less
-// (`lanes` of the 32 carry one).
+// (`lanes` of the 32 carry one).  The vote per bounce brings the lanes together:
+// without it those whose bounce cast no shadow ray ran ahead into the next one
+// (65,536 paths at 32 a warp, mixed scene 534 -> 432 us, Cornell box 158 -> 129).
+// The first `tiled` pixels of the range are walked in 8x4 tiles (seg_pixel), the
+// rest in rows: 2.17M triangles 0-7% faster, the others within 3%.
 constexpr int kPathStack = 8;   // stack entries per thread in shared memory
 
 template <bool F32>
-__global__ void __maxnreg__(96) path_kernel(RenderParams P, uint32_t pixel0, uint32_t n, uint32_t lanes,
+__global__ void __maxnreg__(96) path_kernel(RenderParams P, WaveSeg sg, uint32_t n, uint32_t tiled, uint32_t lanes,
                                             float4* __restrict__ color) {
     __shared__ uint2 stack_sh[kPathStack * 32];
     StackSpill overflow;
     Stack st(stack_sh, overflow, 32, kPathStack);
     const uint32_t i = blockIdx.x * lanes + threadIdx.x;
     uint32_t n_ext = 0, n_shadow = 0;
-    if (threadIdx.x < lanes && i < n) {
-        const uint32_t k = i / P.nspp, pixel = pixel0 + k;
-        PathState ps;
-        Ray ray;
-        begin_path(P.cam, P.seed, P.view, pixel % P.width, pixel / P.width, pixel, P.spp0 + (i - k * P.nspp), ps, ray);
-        while (path_bounce<F32>(P, ps, ray, st, n_ext, n_shadow)) {
+    bool alive = threadIdx.x < lanes && i < n;
+    const bool mine = alive;
+    PathState ps;
+    Ray ray;
+    if (alive) {
+        uint32_t k = i / P.nspp, sample = i - k * P.nspp, pixel = sg.p0 + k;
+        if (k < tiled) {
+            seg_slot_inv(sg, i, k, sample);
+            pixel = seg_pixel(sg, k);
         }
-        color[i] = make_float4(ps.color.x, ps.color.y, ps.color.z, 0.f);
+        begin_path(P.cam, P.seed, P.view, pixel % P.width, pixel / P.width, pixel, P.spp0 + sample, ps, ray);
     }
+    while (__any_sync(0xFFFFFFFFu, alive))
+        if (alive) alive = path_bounce<F32>(P, ps, ray, st, n_ext, n_shadow);
+    if (mine) color[i] = make_float4(ps.color.x, ps.color.y, ps.color.z, 0.f);
     count_rays(P.ray_counts, n_ext, n_shadow);
 }
 
-__global__ void path_sum_kernel(RenderParams P, uint32_t pixel0, uint32_t pixels, const float4* __restrict__ color) {
+__global__ void path_sum_kernel(RenderParams P, WaveSeg sg, uint32_t pixels, uint32_t tiled,
+                                const float4* __restrict__ color) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= pixels) return;
-    float4 acc = P.accum[pixel0 + k];
+    const uint32_t pixel = k < tiled ? seg_pixel(sg, k) : sg.p0 + k;
+    float4 acc = P.accum[pixel];
     for (uint32_t s = 0; s < P.nspp; ++s) {
-        const float4 c = color[(size_t)k * P.nspp + s];
+        const float4 c = color[k < tiled ? seg_slot(sg, k, s) : k * P.nspp + s];
         acc.x = acc.x + c.x;
         acc.y = acc.y + c.y;
         acc.z = acc.z + c.z;
     }
-    P.accum[pixel0 + k] = acc;
+    P.accum[pixel] = acc;
 }
 
 // Queues samples [P.spp0, P.spp0 + P.nspp) of pixels [pixel0, pixel0 + pixels):
 // pixels * nspp paths; `color` holds one float4 per path.
 //
-// Paths per warp: as few as keep the warps near what the chip holds at once
-// (20 per SM at 96 registers, 3,040), which halves the divergence a warp pays
-// for.  Measured with 32 / 16 / 8 / 4 / 2 / 1 paths per warp, mixed scene, us: 65,536
-// paths 519 / 426 / 471 / 533 / 683 / 877, 16,384 paths 414 / 331 / 294 / 234 / 263 /
-// 275, 2,048 paths 383 / 323 / 245 / 190 / 154 / 126.
+// Paths per warp: as few as leave all warps resident at once (20 per SM at 96
+// registers, 3,040).  Measured with 32 / 16 / this many (22) of 65,536 paths, us:
+// mixed scene 256x256 x 1 432 / 545 / 426, 256x64 x 4 382 / 345 / 359; 2.17M
+// triangles 342 / 307 / 326, 377 / 317 / 329; Cornell box 129 / 197 / 138, 105 / 117 /
+// 108.  16,384 paths, mixed scene, 32 / 16 / 8 / 4 / 2 / 1 a warp: 414 / 331 / 294 / 234 /
+// 263 / 275; 2,048 paths 383 / 323 / 245 / 190 / 154 / 126.
 static void launch_paths(const RenderParams& P, bool f32, uint32_t pixel0, uint32_t pixels, float4* color,
                          cudaStream_t s) {
     static const int room[2] = {persistent_grid((const void*)path_kernel<false>, 32, 0),
                                 persistent_grid((const void*)path_kernel<true>, 32, 0)};
-    const uint32_t n = pixels * P.nspp, most = (uint32_t)room[f32] * 11u / 8u;
-    uint32_t lanes = 32;
-    while (lanes > 1 && (n - 1) / (lanes / 2) + 1 <= most) lanes /= 2;
-    (f32 ? path_kernel<true> : path_kernel<false>)<<<(n - 1) / lanes + 1, 32, 0, s>>>(P, pixel0, n, lanes, color);
-    path_sum_kernel<<<(pixels - 1) / 256 + 1, 256, 0, s>>>(P, pixel0, pixels, color);
+    const uint32_t n = pixels * P.nspp, lanes = std::min(32u, (n - 1) / (uint32_t)room[f32] + 1);
+    const uint32_t band = pixel0 % P.width || P.width % 8u ? 0u : 4u * P.width;
+    const uint32_t tiled = band ? pixels / band * band : 0u;
+    const WaveSeg sg{0u, pixel0, pixel0 + pixels, P.spp0, P.spp0 + P.nspp, 0u, 0u, band};
+    (f32 ? path_kernel<true> : path_kernel<false>)<<<(n - 1) / lanes + 1, 32, 0, s>>>(P, sg, n, tiled, lanes, color);
+    path_sum_kernel<<<(pixels - 1) / 256 + 1, 256, 0, s>>>(P, sg, pixels, tiled, color);
 }
 
-// Passes of at most this many paths run on the path kernel.  Wave / path kernel
-// at 65,536 paths: mixed scene 0.96 / 0.63 ms, 2.17M triangles 1.05 / 0.38, Cornell
-// box 0.37 / 0.19; at 262,144: 1.21 / 1.39, 1.45 / 0.74, 0.44 / 0.34.  (And no path
-// state is allocated: a first pass of the wave form allocates gigabytes.)
+// Passes of at most this many paths run on the path kernel.  Wave / path kernel, us:
+// 131,072 paths, mixed scene 755 / 709, 2.17M triangles 937 / 417, Cornell box 265 /
+// 222; 262,144: 982 / 1128, 1119 / 589, 351 / 365; 524,288: 1497 / 2075, 1321 / 893, 498 /
+// 673.  (And no path state is allocated: a first pass of the wave form allocates
+// gigabytes.)
 constexpr uint64_t kDirectPaths = 1u << 17;
 
 // Whether a pass takes the path kernel: a single view, few paths, and no launch
