@@ -1632,12 +1632,12 @@ static AdjointGrids adjoint_grids(crt_render r, const WaveGrids& G) {
     return a;
 }
 
-// The pass's gradient sums added to the caller's.
-__global__ void add_grad_kernel(const double* __restrict__ grad, uint32_t n_mats, float* __restrict__ kd,
-                                float* __restrict__ ka) {
+// The pass's gradient sums added to the caller's arrays, atomically: handles on
+// other streams may be adding to the same ones, and kd and ka may be one array.
+__global__ void add_grad_kernel(const double* __restrict__ grad, uint32_t n_mats, float* kd, float* ka) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < 6u * n_mats; i += gridDim.x * blockDim.x) {
         float* to = i % 6u < 3u ? kd + 3u * (i / 6u) + i % 6u : ka + 3u * (i / 6u) + i % 6u - 3u;
-        *to = (float)((double)*to + grad[i]);
+        atomicAdd(to, (float)grad[i]);
     }
 }
 

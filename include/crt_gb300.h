@@ -454,8 +454,10 @@ CRT_EXPORT int crt_render_view_accum(crt_render r, uint32_t view, float* host_rg
  * block before global atomics.  Always the wavefront form.
  * d_adjoint: device float4 per pixel of every view (the layout of
  * crt_render_accum_device; .w ignored).  d_grad_kd, d_grad_ka: device float
- * [num_materials][3], ADDED to.  At most 1024 materials.  Asynchronous on the
- * handle's stream; the accumulator and sample counts do not change. */
+ * [num_materials][3], ADDED to atomically: handles on different streams may add
+ * to the same arrays, and the two may be one array.  At most 1024 materials.
+ * Asynchronous on the handle's stream; the accumulator and sample counts do not
+ * change. */
 enum { CRT_ADJOINT_EXACT_ROULETTE = 1u };
 CRT_EXPORT int crt_render_adjoint(crt_render r, uint32_t spp0, uint32_t n_spp, const float* d_adjoint,
                                   float* d_grad_kd, float* d_grad_ka, uint32_t flags);
