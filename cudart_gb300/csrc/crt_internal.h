@@ -12,6 +12,7 @@
 #include "../../include/crt_gb300.h"
 #include "bvh8.h"
 #include "crt_device.cuh"
+#include "dev_buf.h"
 
 namespace crt {
 
@@ -32,23 +33,6 @@ struct Arena {
         const size_t here = at;
         at += (bytes + 255) & ~(size_t)255;
         return here;
-    }
-};
-
-// Owning device buffer.
-struct DevBuf {
-    void* p = nullptr;
-    size_t bytes = 0;
-    ~DevBuf() { if (p) cudaFree(p); }
-    cudaError_t alloc(size_t n) {
-        if (p) { cudaFree(p); p = nullptr; }
-        bytes = n;
-        return n ? cudaMalloc(&p, n) : cudaSuccess;
-    }
-    template <typename T> T* as() const { return static_cast<T*>(p); }
-    void swap(DevBuf& o) {
-        std::swap(p, o.p);
-        std::swap(bytes, o.bytes);
     }
 };
 
@@ -79,7 +63,6 @@ struct crt_scene_s {
 // Wavefront path-state buffers (wavefront.cu).
 struct WaveBuffers {
     uint32_t capacity = 0;
-    uint32_t seg_capacity = 0;      // wave segments the segs buffer holds
     bool octant = false;            // queues hold 8 octant regions
     crt::DevBuf ray_o, color, hit, queue_a, queue_b, shadow, shadow_q, counters, waves, segs, prof;
     crt::DevBuf adj_L, adj_W, adj_shadow, adj_hist;   // adjoint replay state, allocated on first use

@@ -150,7 +150,7 @@ int check_device_error(crt_render r) {
 // The handle's staging buffer, at least `bytes` long (work queued on the
 // handle's stream may still use it: freeing the old one waits for that).
 static int ensure_staging(crt_render r, size_t bytes) {
-    if (r->staging.bytes < bytes) CRT_CUDA(r->staging.alloc(bytes));
+    CRT_CUDA(r->staging.reserve(bytes));
     return CRT_OK;
 }
 

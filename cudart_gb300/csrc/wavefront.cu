@@ -1087,8 +1087,7 @@ static int alloc_set(WaveSet& S, uint32_t cap, bool octant, cudaStream_t ready) 
     CRT_CUDA(B.counters.alloc(C_COUNT * 4));
     CRT_CUDA(cudaMemsetAsync(B.counters.p, 0, C_COUNT * 4, ready));
     CRT_CUDA(B.waves.alloc(kMaxWaves * sizeof(uint4)));
-    B.seg_capacity = kMaxWaves;
-    CRT_CUDA(B.segs.alloc((size_t)B.seg_capacity * sizeof(WaveSeg)));
+    CRT_CUDA(B.segs.alloc((size_t)kMaxWaves * sizeof(WaveSeg)));
     CRT_CUDA(B.prof.alloc(P_COUNT * sizeof(unsigned long long)));
     CRT_CUDA(cudaStreamCreateWithFlags(&S.stream, cudaStreamNonBlocking));
     CRT_CUDA(cudaEventCreateWithFlags(&S.acc_done, cudaEventDisableTiming));
@@ -1119,13 +1118,12 @@ static int ensure_wave_sets(crt_render r, uint32_t count) {
 // Room for n segments in a set's table; a larger table invalidates the
 // set's captured graph, which holds the old address.
 static int ensure_segments(WaveSet& set, size_t n) {
-    WaveBuffers& B = set.buf;
-    if (n <= B.seg_capacity) return CRT_OK;
+    DevBuf& segs = set.buf.segs;
+    if (n * sizeof(WaveSeg) <= segs.bytes) return CRT_OK;
     if (n > (size_t)UINT32_MAX) return set_error(CRT_ERR_LIMIT, "too many wave segments");
     CRT_CUDA(cudaStreamSynchronize(set.stream));
     drop_set_graphs(set);
-    B.seg_capacity = (uint32_t)std::max<size_t>(n, 2ull * B.seg_capacity);
-    CRT_CUDA(B.segs.alloc((size_t)B.seg_capacity * sizeof(WaveSeg)));
+    CRT_CUDA(segs.reserve(std::max(n * sizeof(WaveSeg), 2 * segs.bytes)));
     return CRT_OK;
 }
 
@@ -1508,7 +1506,7 @@ int wavefront_pass(crt_render r, const std::vector<ViewWork>& work) {
         const size_t bytes = (size_t)npix * work[0].nspp * sizeof(float4);
         if (r->path_color.bytes < bytes) {
             CRT_CUDA(cudaStreamSynchronize(r->stream));
-            CRT_CUDA(r->path_color.alloc(bytes));
+            CRT_CUDA(r->path_color.reserve(bytes));
         }
         launch_paths(make_params(r, 0, work[0].spp0, work[0].nspp), uses_f32_nodes(r), 0, npix,
                      r->path_color.as<float4>(), r->stream);
