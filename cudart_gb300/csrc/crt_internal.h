@@ -67,7 +67,6 @@ struct WaveBuffers {
     crt::DevBuf ray_o, color, hit, queue_a, queue_b, shadow, shadow_q, counters, waves, segs, prof;
     crt::DevBuf adj_L, adj_W, adj_shadow, adj_hist;   // adjoint replay state, allocated on first use
     crt::DevBuf adj_hits, adj_vis;                    // the primal trace's record (wavefront.cu)
-    bool adj_no_room = false;                         // no memory for the record
 };
 
 // One independent set of wavefront buffers with its own stream and captured
@@ -118,6 +117,7 @@ struct crt_render_s {
     bool own_stream = false;
     crt::DevBuf accum, lut, ray_counts, view_table, staging;
     crt::DevBuf adj_grad;           // gradient sums of an adjoint pass
+    bool adj_no_room = false;       // no memory for the adjoint's records
     crt::DevBuf path_color;         // radiance per path of a pass on the path kernel
     std::vector<WaveSet> sets;
     uint32_t scene_generation = 0;  // scene BVH the captured wave graphs point at

@@ -1579,10 +1579,9 @@ int wavefront_pass(crt_render r, const std::vector<ViewWork>& work) {
 }
 
 // ---------------------------------------------------------------------------
-// Adjoint pass (crt_render_adjoint): every wave is traced twice from the same
-// Philox counters -- the primal trace leaves each path's radiance in st_c,
-// then the replay re-runs the path and turns each event into gradient terms
-// (WaveGrad) -- so nothing per vertex is stored.
+// Adjoint pass (crt_render_adjoint): every wave runs twice from the same Philox
+// counters -- the primal trace leaves each path's radiance in st_cm, then the
+// replay re-runs the path and turns each event into gradient terms (WaveGrad).
 // ---------------------------------------------------------------------------
 // Up to this many bounces the primal trace records each path's hits (16 bytes a
 // bounce) and light visibilities (a bit a bounce), and the replay reads them
@@ -1590,24 +1589,45 @@ int wavefront_pass(crt_render r, const std::vector<ViewWork>& work) {
 constexpr uint32_t kRecordDepth = 16;
 constexpr size_t kRecordBytes = 6ull << 30;   // per wave set
 
-static int ensure_adjoint_buffers(WaveSet& set, bool exact, uint32_t max_depth) {
-    WaveBuffers& B = set.buf;
-    const size_t c = B.capacity;
-    if (!B.adj_L.p) {
-        CRT_CUDA(B.adj_L.alloc(c * 16));
-        CRT_CUDA(B.adj_W.alloc(c * 16));
-        CRT_CUDA(B.adj_shadow.alloc(c * 16));
+static void free_records(crt_render r) {
+    for (WaveSet& set : r->sets) {
+        set.buf.adj_hits.alloc(0);
+        set.buf.adj_vis.alloc(0);
     }
-    if (exact && !B.adj_hist.p) CRT_CUDA(B.adj_hist.alloc(c * kHistMax * sizeof(uint16_t)));
-    if (max_depth <= kRecordDepth && c * 16 * max_depth <= kRecordBytes && !B.adj_hits.p && !B.adj_no_room) {
-        // without room for the record the replay traces its rays again
-        if (B.adj_hits.alloc(c * 16 * max_depth) != cudaSuccess || B.adj_vis.alloc(c * 4) != cudaSuccess) {
-            cudaGetLastError();
-            B.adj_hits.alloc(0);
-            B.adj_vis.alloc(0);
-            B.adj_no_room = true;
+    r->adj_no_room = true;
+}
+
+// The adjoint's buffers: first what it cannot do without, of every set; then the
+// records, if as much memory again is left beside them (other handles and the
+// caller's own work need some).  Without its record the replay traces its rays.
+static int ensure_adjoint_buffers(crt_render r, bool exact) {
+    auto needed = [&]() -> cudaError_t {
+        for (WaveSet& set : r->sets) {
+            WaveBuffers& B = set.buf;
+            const size_t c = B.capacity;
+            cudaError_t e = B.adj_L.reserve(c * 16);
+            if (e == cudaSuccess) e = B.adj_W.reserve(c * 16);
+            if (e == cudaSuccess) e = B.adj_shadow.reserve(c * 16);
+            if (e == cudaSuccess && exact) e = B.adj_hist.reserve(c * kHistMax * sizeof(uint16_t));
+            if (e != cudaSuccess) return e;
         }
+        return r->adj_grad.reserve((size_t)6 * r->scene->n_mats * sizeof(double));
+    };
+    cudaError_t e = needed();
+    if (e != cudaSuccess && r->sets[0].buf.adj_hits.p) {
+        drop_wave_graphs(r);   // waits for the passes that use the records
+        free_records(r);
+        e = needed();
     }
+    CRT_CUDA(e);
+    const size_t c = r->sets[0].buf.capacity, hits = c * 16 * r->opts.max_depth, vis = c * 4;
+    if (r->opts.max_depth > kRecordDepth || hits > kRecordBytes || r->adj_no_room || r->sets[0].buf.adj_hits.p)
+        return CRT_OK;
+    size_t left = 0, total = 0;
+    bool room = cudaMemGetInfo(&left, &total) == cudaSuccess && left / 2 >= r->sets.size() * (hits + vis);
+    for (WaveSet& set : r->sets)
+        room = room && set.buf.adj_hits.alloc(hits) == cudaSuccess && set.buf.adj_vis.alloc(vis) == cudaSuccess;
+    if (!room) free_records(r);
     return CRT_OK;
 }
 
@@ -1717,11 +1737,8 @@ int wavefront_adjoint(crt_render r, const std::vector<ViewWork>& work, const flo
     const uint32_t K = r->opts.wave_sets ? r->opts.wave_sets : kDefaultWaveSets;
     int st = ensure_wave_sets(r, K);
     if (st != CRT_OK) return st;
-    for (WaveSet& s : r->sets)
-        if ((st = ensure_adjoint_buffers(s, exact, r->opts.max_depth)) != CRT_OK) return st;
-    const size_t grad_bytes = (size_t)6 * r->scene->n_mats * sizeof(double);
-    if (!r->adj_grad.p) CRT_CUDA(r->adj_grad.alloc(grad_bytes));   // a scene keeps its material count
-    CRT_CUDA(cudaMemsetAsync(r->adj_grad.p, 0, grad_bytes, r->stream));
+    if ((st = ensure_adjoint_buffers(r, exact)) != CRT_OK) return st;
+    CRT_CUDA(cudaMemsetAsync(r->adj_grad.p, 0, r->adj_grad.bytes, r->stream));   // a scene keeps its material count
     const uint32_t cap = r->sets[0].buf.capacity;
     const WavePlan plan = make_waves(r, work, cap);
     if (r->scene_generation != r->scene->generation) {

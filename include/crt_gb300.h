@@ -441,9 +441,13 @@ CRT_EXPORT int crt_render_view_accum(crt_render r, uint32_t view, float* host_rg
  * material's kd (diffuse albedo; diffuse vertices of untextured materials)
  * and ka (emission as given in crt_material).  For an image loss L(I) with
  * I = accum / spp, pass adjoint = dL/dI / spp.
- * Path-replay backpropagation: each path is traced twice from the same
- * Philox counters, first for its radiance, then again turning every vertex
- * into gradient terms, so nothing per vertex is stored.  By default Russian
+ * Path-replay backpropagation: each path runs twice from the same Philox
+ * counters, first for its radiance, then again turning every vertex into
+ * gradient terms.  Up to 16 bounces the first run records each path's hits and
+ * light visibilities (16 bytes a path and bounce, at most 6 GiB per wave set,
+ * kept by the handle: 17 GB at 1080p and depth 8) and the second reads them;
+ * beyond that, or where the device has not twice the record's memory free, the
+ * second traces the same rays again.  By default Russian
  * roulette's survival probability counts as a constant: the gradient is
  * unbiased for the expected image (roulette is unbiased whatever the
  * probability).  CRT_ADJOINT_EXACT_ROULETTE also differentiates the
