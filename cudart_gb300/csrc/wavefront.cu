@@ -862,6 +862,10 @@ static WaveKernel shadow_kernel(uint32_t flags, bool f32) {
 
 __global__ void wf_flip(WaveParams W) {
     const uint32_t cur = W.counters[C_CUR];
+    if (W.vis) {   // the adjoint's recorded trace: the replay's rays of this bounce, read back instead of traced
+        atomicAdd(W.R.ray_counts, (unsigned long long)W.counters[cur]);
+        atomicAdd(W.R.ray_counts + 1, (unsigned long long)W.counters[C_SHADOW]);
+    }
     W.counters[cur] = 0;
     if (W.octant) {
         uint32_t total = 0;

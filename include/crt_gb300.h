@@ -505,7 +505,8 @@ CRT_EXPORT int crt_render_tile_noalloc(crt_scene scene, const crt_camera* camera
                                        uint32_t pixel0, uint32_t pixel_count, uint32_t spp0,
                                        uint32_t nspp, float* d_accum, void* stream);
 
-/* Extension and shadow rays traced by the passes since the last reset. */
+/* Extension and shadow rays of the passes since the last reset.  An adjoint pass
+ * counts both of its traces, whether the second traced its rays or read them. */
 CRT_EXPORT int crt_render_ray_counts(crt_render r, uint64_t* extension_rays, uint64_t* shadow_rays);
 
 /* ---- autotuner ------------------------------------------------------
