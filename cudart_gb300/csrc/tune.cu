@@ -11,7 +11,8 @@
 // others held, and a value is adopted when it beats the current best by more
 // than the noise margin.  Every candidate renders the same samples (a fresh
 // handle from sample 0), timed with CUDA events on the handle's stream after
-// one untimed pass that allocates and captures its wave graphs.
+// one untimed pass that allocates and captures its wave graphs.  Every candidate
+// names its wave size, so all of them run the wave form, however few their paths.
 #include <algorithm>
 #include <chrono>
 #include <cstring>
@@ -243,6 +244,9 @@ int crt_autotune(crt_scene scene, const crt_camera* camera, uint32_t width, uint
             return st;
         }
     }
+    // a wave size that is the default's is left to the default, so that passes of
+    // few paths may run on the path kernel
+    if (!o.wave_paths && best.wave_paths == default_wave_paths((uint64_t)width * height)) best.wave_paths = 0;
     std::memset(out, 0, sizeof(*out));
     out->options = best;
     out->bvh_width = best_width;

@@ -1489,13 +1489,11 @@ static void launch_paths(const RenderParams& P, bool f32, uint32_t pixel0, uint3
 // gigabytes.)
 constexpr uint64_t kDirectPaths = 1u << 17;
 
-// Whether a pass takes the path kernel: a single view, few paths, and no launch
-// shape asked for (an explicit wave size, set count, block size and so on is the
-// caller's choice of the wavefront form).
+// Whether a pass takes the path kernel: a single view, few paths, and the wave
+// form not asked for by a wave size or a scheduling flag.  (Block size, stack
+// depth, queue chunk and set count shape the wave form where it runs.)
 static bool direct_pass(crt_render r, const std::vector<ViewWork>& work) {
-    const crt_render_options& o = r->opts;
-    if (work.size() != 1 || o.wave_paths || o.wave_sets || o.flags || o.block_size || o.stack_depth || o.queue_chunk)
-        return false;
+    if (work.size() != 1 || r->opts.wave_paths || r->opts.flags) return false;
     return (uint64_t)r->views[0].npix() * work[0].nspp <= kDirectPaths;
 }
 

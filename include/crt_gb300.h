@@ -266,9 +266,10 @@ CRT_EXPORT int crt_measure_gather(const void* d_buf, uint64_t bytes, uint32_t re
 typedef enum {
     CRT_MODE_MEGAKERNEL = 0,   /* one kernel per pass runs whole paths */
     CRT_MODE_WAVEFRONT = 1     /* generate / extend / shade / shadow queues; a
-                                  single-view pass of at most 2^17 paths whose
-                                  launch options are all default runs each path in
-                                  one thread instead (1.5 to 5 times faster there) */
+                                  single-view pass of at most 2^17 paths on a handle
+                                  with neither wave_paths nor flags set runs each
+                                  path in one thread instead (four scenes: 1.1 to
+                                  2.3 times faster at 2^17 paths, 2.8 to 5 at 2^11) */
 } crt_mode;
 
 /* Traversal scheduling of the wavefront's persistent kernels.  The default
@@ -396,7 +397,9 @@ typedef struct {
  * with the wavefront stages launched one by one instead of through the
  * graph, each timed with CUDA events on the handle's stream; every
  * extension and shadow traversal is re-run untimed in counting mode to
- * report node visits and triangle tests.  Wavefront handles only. */
+ * report node visits and triangle tests.  Wavefront handles only; always the
+ * wave stages, also for a pass of so few paths that crt_render_pass would not
+ * run them (crt_mode). */
 CRT_EXPORT int crt_render_profile_pass(crt_render r, uint32_t n_spp, crt_stage_profile* out);
 
 /* ---- batched views ------------------------------------------------------
@@ -516,7 +519,8 @@ CRT_EXPORT int crt_render_ray_counts(crt_render r, uint64_t* extension_rays, uin
  * searches, by coordinate descent, the options that change speed but not
  * the image: node_format, block_size, stack_depth, queue_chunk, wave_sets,
  * wave_paths, CRT_FLAG_LANE_REFILL and (tune_bvh_width) the BVH
- * width.
+ * width.  All trials run the wave queues, also where a pass has so few paths
+ * that it would not by default (crt_mode).
  * The device must be otherwise idle for the timings to mean anything.  With
  * tune_bvh_width the scene's BVH is rebuilt (crt_scene_set_bvh_width) and
  * the faster width is left in place. */
@@ -530,7 +534,10 @@ typedef struct {
 } crt_tune_params;
 
 typedef struct {
-    crt_render_options options;  /* fastest options (mode = wavefront, defaults spelled out) */
+    crt_render_options options;  /* fastest options of the wave form (mode = wavefront,
+                                    defaults spelled out; wave_paths stays 0 where its
+                                    default was not beaten, so that with no flag set
+                                    passes of few paths take the form of crt_mode) */
     uint32_t bvh_width;          /* BVH width left in the scene */
     uint32_t candidates;         /* distinct candidates timed */
     float ms_per_spp;            /* fastest: milliseconds per sample per pixel */
