@@ -90,7 +90,8 @@ inline uint32_t plane16(double v, bool hi, bool high_half) {
     if (hi) {
         while (value(h << 16) < v) ++h;
     } else {
-        while (h > 0 && value((h << 16) | (high_half ? 0xFFFFu : 0u)) > v) --h;
+        // (not above v, and a number: past FLT_MAX a high half would read as infinite or NaN)
+        while (h > 0 && !(value((h << 16) | (high_half ? 0xFFFFu : 0u)) <= v)) --h;
     }
     return h;
 }
