@@ -617,20 +617,16 @@ def run_gb300(args):
         peak, peak_kind = measured_peaks()
         node_bytes = NODE_BYTES if wf.options.node_format != 1 else F32_NODE_BYTES
         roof = {}
-        # algorithmic bytes of the gathers (visits to nodes staged in shared
-        # memory, none with this library, would be counted apart)
-        for stage, rays, nodes, tris, top in (
-                ("extend", "extension_rays", "extension_nodes", "extension_tris", "extension_top_nodes"),
-                ("shadow", "shadow_rays", "shadow_nodes", "shadow_tris", "shadow_top_nodes")):
+        # algorithmic bytes of the gathers
+        for stage, rays, nodes, tris in (("extend", "extension_rays", "extension_nodes", "extension_tris"),
+                                         ("shadow", "shadow_rays", "shadow_nodes", "shadow_tris")):
             launches = prof[f"{stage}_launches"]
-            alg = (prof[nodes] - prof[top]) * node_bytes + prof[tris] * TRI_BYTES
+            alg = prof[nodes] * node_bytes + prof[tris] * TRI_BYTES
             ms_l = prof[f"{stage}_ms"] / launches
             gbs = alg / launches / (ms_l * 1e-3) / 1e9
             roof[stage] = {"kernel": "wf_" + stage, "bytes_per_launch": alg / launches,
                            "ms_per_launch": ms_l, "gbs": gbs, "rays": prof[rays],
                            "nodes_per_ray": prof[nodes] / max(prof[rays], 1),
-                           "staged_nodes_per_ray": prof[top] / max(prof[rays], 1),
-                           "shared_memory_bytes_per_launch": prof[top] * node_bytes / launches,
                            "tris_per_ray": prof[tris] / max(prof[rays], 1)}
         main = roof["extend"] if dom != "shadow" else roof["shadow"]
         traffic = None
@@ -647,8 +643,7 @@ def run_gb300(args):
         # L1 sector hit rate (ncu, profiles/wf_extend_cache.json):
         # 1 / (h1 / BW_L1 + (1 - h1) / BW_L2), weighted by the byte mix
         ext_k = main["kernel"] == "wf_extend"
-        nb = (prof["extension_nodes" if ext_k else "shadow_nodes"]
-              - prof["extension_top_nodes" if ext_k else "shadow_top_nodes"]) * node_bytes
+        nb = prof["extension_nodes" if ext_k else "shadow_nodes"] * node_bytes
         tb = prof["extension_tris" if ext_k else "shadow_tris"] * TRI_BYTES
         g1 = gather_ceiling(torch, stream, [GATHER_BYTES[b] for b in (node_bytes, TRI_BYTES)], working_set=96 << 10, l1=True)
         g2 = gather_ceiling(torch, stream, [GATHER_BYTES[b] for b in (node_bytes, TRI_BYTES)], working_set=64 << 20, l1=True)
@@ -676,16 +671,13 @@ def run_gb300(args):
                     "limiter": "L1 data pipe and issue at half the lanes: see profiles/wf_extend_large_textured_1080p.md; "
                                "lanes of a warp in one node share its loads, so frac may pass 1",
                     "algorithmic_bytes": f"nodes visited x {node_bytes} B "
-                                         "+ triangles tested x 40 B per ray",
-                    "staged_nodes_per_ray": round(main["staged_nodes_per_ray"], 3)}
+                                         "+ triangles tested x 40 B per ray"}
         l2_peak = hier
         step_bytes = None
         if main["kernel"] == "wf_extend":
             # per-step cross-check: all traversal bytes of a step / its time
-            per_ray_ext = ((roof["extend"]["nodes_per_ray"] - roof["extend"]["staged_nodes_per_ray"]) * node_bytes
-                           + roof["extend"]["tris_per_ray"] * TRI_BYTES)
-            per_ray_shd = ((roof["shadow"]["nodes_per_ray"] - roof["shadow"]["staged_nodes_per_ray"]) * node_bytes
-                           + roof["shadow"]["tris_per_ray"] * TRI_BYTES)
+            per_ray_ext = roof["extend"]["nodes_per_ray"] * node_bytes + roof["extend"]["tris_per_ray"] * TRI_BYTES
+            per_ray_shd = roof["shadow"]["nodes_per_ray"] * node_bytes + roof["shadow"]["tris_per_ray"] * TRI_BYTES
             step_bytes = ext * per_ray_ext + shd * per_ray_shd
             roofline["step_check"] = {"traversal_bytes_per_step": round(step_bytes),
                                       "gbs_over_whole_step": round(step_bytes / (ms_step * 1e-3) / 1e9, 1),
@@ -793,7 +785,7 @@ def run_gb300(args):
                                    "seconds_per_step")}
         detail["roofline_line"] = dict(roofline)
         roofline = {k: roofline[k] for k in ("bound", "kernel", "achieved", "peak", "unit", "frac",
-                                             "traffic", "l2_only", "hbm", "step_check", "staged_nodes_per_ray")
+                                             "traffic", "l2_only", "hbm", "step_check")
                     if k in roofline}
         roofline["hbm"] = {k: roofline["hbm"][k] for k in ("achieved", "peak", "frac")}
         if c4:

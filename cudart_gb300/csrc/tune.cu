@@ -26,12 +26,11 @@ namespace {
 
 constexpr float kAdoptMargin = 0.02f;   // a candidate must be 2 % faster to move the search
 
-using Key = std::tuple<int32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t,
-                       uint32_t>;
+using Key = std::tuple<int32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t>;
 
 Key key_of(const crt_render_options& o, uint32_t bvh_width) {
     return Key(o.node_format, o.block_size, o.stack_depth, o.queue_chunk, o.wave_sets, o.wave_paths,
-               o.flags, o.top_nodes, o.refill_busy, bvh_width);
+               o.flags, o.refill_busy, bvh_width);
 }
 
 struct Tuner {
