@@ -239,7 +239,7 @@ CRT_D void zero_grad_block(float* acc, uint32_t n_mats) {
 }
 
 // A block's sums into the pass's, in FP64: some 60,000 blocks and bounces add to
-// each material, and their FP32 sum was off by 6-8e-6 of the gradient (now 1e-6).
+// each material, and their FP32 sum was off by 7-9e-6 of the gradient (now 2-7e-8).
 CRT_D void flush_grad_block(const WaveParams& W, const float* acc) {
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < 6u * W.n_mats; i += blockDim.x) {
@@ -1878,7 +1878,7 @@ int wavefront_profile_pass(crt_render r, const std::vector<ViewWork>& work, crt_
 //
 // The wavefront form's four launches per bounce cost a 64K-path tile 918 us
 // (mixed scene, depth 8; 1,104 us before the node layouts): every bounce waited
-// for its slowest ray.  The path kernel takes 415 us.
+// for its slowest ray.  The path kernel takes 377 us.
 // ---------------------------------------------------------------------------
 Camera to_device_camera(const crt_camera& c);
 

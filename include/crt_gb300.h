@@ -142,7 +142,7 @@ typedef enum {
 /* BVH node encoding on the device (same tree, same results either way). */
 typedef enum {
     CRT_NODES_Q8 = 0,    /* quantised nodes: child planes as 16-bit floats relative to
-                            the node, rounded outward; 160 bytes apart, 120 read.  The
+                            the node, rounded outward; 160 bytes apart, 128 read.  The
                             faster one on every workload measured */
     CRT_NODES_F32 = 1    /* 208-byte nodes with FP32 child planes */
 } crt_node_format;
@@ -273,11 +273,12 @@ typedef enum {
 } crt_mode;
 
 /* Traversal scheduling of the wavefront's persistent kernels.  The default
- * (0): a warp takes 32 rays and finishes them all before taking more, and a
- * node visit tests all triangles of the leaves it hits. */
+ * (0): a warp takes 32 rays and finishes them all before taking more, unless its
+ * first ones differ so widely in length that it goes over to refilling idle lanes,
+ * and a node visit tests all triangles of the leaves it hits. */
 enum {
-    CRT_FLAG_LANE_REFILL = 1u,  /* a lane whose ray finished takes the next one
-                                   at once (warp-local pool of queue entries) */
+    CRT_FLAG_LANE_REFILL = 1u,  /* lanes whose rays finished take the queue's next
+                                   ones (refill_busy says when) */
     CRT_FLAG_SPLIT_LEAF = 2u,   /* one triangle test per traversal step, so lanes
                                    in leaves and lanes in inner nodes interleave */
     CRT_FLAG_OCTANT_QUEUES = 4u, /* shade files surviving paths by the octant of
@@ -477,8 +478,7 @@ CRT_EXPORT int crt_render_adjoint(crt_render r, uint32_t spp0, uint32_t n_spp, c
  * cudaMalloc / cudaFree and the device synchronisation they cause.
  *
  * Renders samples [spp0, spp0 + nspp) of the pixels [pixel0, pixel0 +
- * pixel_count) of a width x height image with the wavefront kernels and
- * adds each pixel's per-sample radiance, in sample order, to d_accum[pixel]
+ * pixel_count) of a width x height image, each path in one thread, and adds each pixel's per-sample radiance, in sample order, to d_accum[pixel]
  * (the caller's device buffer of width*height x 4 floats: rgb + unused,
  * 16-byte aligned; same layout as crt_render_accum_device).  Sums are
  * bit-identical to crt_render_pass when calls cover each pixel's samples in
